@@ -14,7 +14,7 @@
 // identical LM decisions.  The Gauss-Newton normal equations J^T J, J^T r are contracted on the
 // FP64 tensor cores (mma.sync m8n8k4 .f64) from Jacobian rows staged in a per-warp
 // shared-memory tile, and kept there between LM steps; the damped system is solved in FP64
-// with its rows spread over lanes.  Warps of a block take voxels from a shared counter.
+// with its rows spread over lanes.  Warps take voxels from a launch-wide counter.
 //
 // Precision: everything is FP64 -- parameters, model values, residuals, cost, gradient and the
 // Gauss-Newton Hessian.  The reference's CPU fits are FP64, and on near-singular fits (a small
@@ -968,8 +968,7 @@ __device__ __forceinline__ Real predict_final(int model, const Real* q, int o, b
 //   C  the f0 re-fit of the voxels the plausibility rule flags (CUDA/xfibres_gpu.cu:207-339)
 //   D  tau = 1/var(residuals) and the FP32 outputs
 // Between stages each voxel's FP64 parameters stay in scratch ([nvox][16] doubles) and its
-// state in a flag word.  One warp per voxel; the warps of a block take voxels from a
-// shared-memory counter.
+// state in a flag word.  One warp per voxel; the warps of the grid take voxels from a counter.
 // ------------------------------------------------------------------------------------------
 // kFitCapped: the LM run that produced the voxel's current parameters stopped at its iteration cap
 enum FitFlag : uint32_t { kFitBad = 1u, kFitRefit = 2u, kFitRefitted = 4u, kFitCapped = 8u };
@@ -1153,44 +1152,43 @@ __device__ void stage_finish(const FitArgs& a, int v, int lane, double*) {
     a.status[v] = (refit ? BPX_VOX_F0_REFIT : 0u) | ((flag & kFitCapped) ? BPX_VOX_LM_ITERATION_CAP : 0u);
 }
 
-// Each block owns kFitVoxPerBlock consecutive voxels; its warps take the next one from a
-// shared-memory counter as they finish, so a voxel whose fit runs 200 iterations holds up one
-// warp instead of a fixed share of the block's voxels.
+// The warps of a resident grid take voxels from the launch's counter (queue, zero before it) as they
+// finish, so a voxel whose fit runs 200 iterations holds up one warp and a volume of any size spreads
+// over every SM.  (With 32 consecutive voxels shared out inside each block, a volume of a few
+// thousand voxels left SMs idle or doubly loaded: 8192 / 12800 whole-brain voxels took 206 / 245 ms,
+// with the launch-wide counter 133 / 187 ms.)
 template <typename Stage>
-__device__ __forceinline__ void run_stage(const FitArgs& a, Stage stage) {
+__device__ __forceinline__ void run_stage(const FitArgs& a, unsigned int* queue, Stage stage) {
   __shared__ double stage_buf[kFitThreads / 32][kStageDoubles];
-  __shared__ int next;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int warps = gridDim.x * (kFitThreads / 32);
   double* st = stage_buf[w];
   for (int i = lane; i < kStageDoubles; i += 32) st[i] = 0.0;
-  const int v0 = blockIdx.x * kFitVoxPerBlock;
-  const int v1 = min(v0 + kFitVoxPerBlock, a.nvox);
-  if (threadIdx.x == 0) next = v0 + kFitThreads / 32;
-  __syncthreads();
-  int v = v0 + w;
-  while (v < v1) {
+  __syncwarp();
+  int v = blockIdx.x * (kFitThreads / 32) + w;
+  while (v < a.nvox) {
     stage(a, v, lane, st);
-    int nv = 0;
-    if (lane == 0) nv = atomicAdd(&next, 1);
-    v = __shfl_sync(0xffffffffu, nv, 0);
+    unsigned int n = 0;
+    if (lane == 0) n = atomicAdd(queue, 1u);
+    v = warps + (int)__shfl_sync(0xffffffffu, n, 0);
   }
 }
 
 template <int K, bool F0>
-__global__ void __launch_bounds__(kFitThreads, kFitMinBlocks) fit_start_kernel(FitArgs a) {
-  run_stage(a, [](const FitArgs& x, int v, int lane, double* st) { stage_start<K, F0>(x, v, lane, st); });
+__global__ void __launch_bounds__(kFitThreads, kFitMinBlocks) fit_start_kernel(FitArgs a, unsigned int* queue) {
+  run_stage(a, queue, [](const FitArgs& x, int v, int lane, double* st) { stage_start<K, F0>(x, v, lane, st); });
 }
 template <int K, bool F0>
-__global__ void __launch_bounds__(kFitThreads, kFitMinBlocks) fit_multi_kernel(FitArgs a) {
-  run_stage(a, [](const FitArgs& x, int v, int lane, double* st) { stage_multi<K, F0>(x, v, lane, st); });
+__global__ void __launch_bounds__(kFitThreads, kFitMinBlocks) fit_multi_kernel(FitArgs a, unsigned int* queue) {
+  run_stage(a, queue, [](const FitArgs& x, int v, int lane, double* st) { stage_multi<K, F0>(x, v, lane, st); });
 }
 template <int K>
-__global__ void __launch_bounds__(kFitThreads, kFitMinBlocks) fit_refit_kernel(FitArgs a) {
-  run_stage(a, [](const FitArgs& x, int v, int lane, double* st) { stage_refit<K>(x, v, lane, st); });
+__global__ void __launch_bounds__(kFitThreads, kFitMinBlocks) fit_refit_kernel(FitArgs a, unsigned int* queue) {
+  run_stage(a, queue, [](const FitArgs& x, int v, int lane, double* st) { stage_refit<K>(x, v, lane, st); });
 }
 template <int K, bool F0>
-__global__ void __launch_bounds__(kFitThreads, kFitMinBlocks) fit_finish_kernel(FitArgs a) {
-  run_stage(a, [](const FitArgs& x, int v, int lane, double* st) { stage_finish<K, F0>(x, v, lane, st); });
+__global__ void __launch_bounds__(kFitThreads, kFitMinBlocks) fit_finish_kernel(FitArgs a, unsigned int* queue) {
+  run_stage(a, queue, [](const FitArgs& x, int v, int lane, double* st) { stage_finish<K, F0>(x, v, lane, st); });
 }
 
 // remove_NonPositive_entries (CUDA/xfibres_gpu.cu:350-367), one warp per voxel
@@ -1220,14 +1218,29 @@ __global__ void __launch_bounds__(kFitThreads) prepare_kernel(int nvox, int ndir
 // ------------------------------------------------------------------------------------------
 // launchers
 // ------------------------------------------------------------------------------------------
+// One stage over every voxel: as many blocks as fit the device at once, fewer for small volumes.
+static cudaError_t launch_stage(void (*kern)(FitArgs, unsigned int*), const FitArgs& a, unsigned int* queue,
+                                cudaStream_t s) {
+  int per_sm = 0;
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFitThreads, 0);
+  if (e != cudaSuccess) return e;
+  const int cap = sm_count() * (per_sm > 0 ? per_sm : 1), warps = kFitThreads / 32;
+  const int want = (int)(((long long)a.nvox + warps - 1) / warps);
+  kern<<<want < cap ? want : cap, kFitThreads, 0, s>>>(a, queue);
+  return cudaGetLastError();
+}
+
 template <int K, bool F0>
 static cudaError_t launch_fit_kf(const FitArgs& a, cudaStream_t s) {
-  const int grid = (a.nvox + kFitVoxPerBlock - 1) / kFitVoxPerBlock;
-  fit_start_kernel<K, F0><<<grid, kFitThreads, 0, s>>>(a);
-  if (a.model >= 2) fit_multi_kernel<K, F0><<<grid, kFitThreads, 0, s>>>(a);
-  if (F0) fit_refit_kernel<K><<<grid, kFitThreads, 0, s>>>(a);
-  fit_finish_kernel<K, F0><<<grid, kFitThreads, 0, s>>>(a);
-  return cudaGetLastError();
+  // the stages' voxel counters take the last two of voxel 0's 16 scratch doubles, which no stage uses
+  static_assert(LmShape<kMulti, K, F0>::P <= 14, "scratch doubles 14 and 15 hold the voxel counters");
+  unsigned int* queue = reinterpret_cast<unsigned int*>(a.scratch + 14);
+  cudaError_t e = cudaMemsetAsync(queue, 0, 4 * sizeof(unsigned int), s);
+  if (e == cudaSuccess) e = launch_stage(fit_start_kernel<K, F0>, a, queue, s);
+  if (e == cudaSuccess && a.model >= 2) e = launch_stage(fit_multi_kernel<K, F0>, a, queue + 1, s);
+  if (e == cudaSuccess && F0) e = launch_stage(fit_refit_kernel<K>, a, queue + 2, s);
+  if (e == cudaSuccess) e = launch_stage(fit_finish_kernel<K, F0>, a, queue + 3, s);
+  return e;
 }
 
 cudaError_t launch_fit(const FitArgs& a, int nfib, bool f0, cudaStream_t s) {

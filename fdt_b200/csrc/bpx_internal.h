@@ -20,7 +20,6 @@ struct NvtxRange {
 };
 
 constexpr int kFitThreads = 128;   // 4 warps, one voxel per warp at a time
-constexpr int kFitVoxPerBlock = 32;  // voxels a fit block shares out among its warps
 #ifndef BPX_FIT_MIN_BLOCKS
 #define BPX_FIT_MIN_BLOCKS 4
 #endif
@@ -77,7 +76,9 @@ struct FitArgs {
   uint32_t* status;
   int model, rician, nonlin;
   float R;
-  double* scratch;   // [nvox][16] FP64 parameters between the fit stages (kFitScratchBytes per voxel)
+  // [nvox][16] FP64 parameters between the fit stages (kFitScratchBytes per voxel); the last two doubles
+  // of voxel 0 hold the stages' voxel counters
+  double* scratch;
   uint32_t* flags;   // [nvox] stage flags (within kFitScratchBytes)
 };
 constexpr size_t kFitScratchBytes = 16 * sizeof(double) + sizeof(uint32_t);  // per voxel
