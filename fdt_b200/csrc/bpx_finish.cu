@@ -4,8 +4,13 @@
 // (CUDA/xfibres_gpu.cu:659-738, CUDA/samples.cu:134-347), which the reference runs on the host
 // after copying every record back: per voxel the sample means, the principal eigenvector of
 // each fibre's mean dyadic tensor, and the fibres re-ordered by decreasing sum of f over samples
-// into the th/ph/f sample arrays.  One thread per voxel; the [row][sample][voxel] layout makes
-// every read and write coalesced across a warp.
+// into the th/ph/f sample arrays.
+//
+// Layout: a block takes 32 voxels, its eight warps every eighth sample of them, so each row of a
+// sample is one 128-byte line and 64K voxels (or 500) put eight times as many loads in flight as one
+// thread per voxel walking all samples would; that serial walk, not HBM, bounded the first form (65536
+// voxels x 50 samples, 3 fibres: 439 us for finishing and 246 us for the post-processing maps).  The
+// warps' FP64 partial sums are added in warp order, so a run reproduces.
 #include <cstdint>
 
 #include "bpx_device.cuh"
@@ -64,19 +69,79 @@ __device__ double principal_vector(double (&A)[3][3], double (&out)[3]) {
   return A[best][best];
 }
 
+constexpr int kVox = 32, kGroups = 8;  // voxels and sample groups (warps) of a block
+
+// Sums over the block's sample groups of Q quantities per voxel: fin[q][voxel] on return (synchronised).
+template <int Q>
+__device__ __forceinline__ void sum_groups(const double (&val)[Q], double (*fin)[kVox]) {
+  __shared__ double buf[kGroups][kGroups][kVox];
+  const int x = threadIdx.x, g = threadIdx.y;
+#pragma unroll
+  for (int q0 = 0; q0 < Q; q0 += kGroups) {
+#pragma unroll
+    for (int q = 0; q < kGroups; ++q)
+      if (q0 + q < Q) buf[g][q][x] = val[q0 + q];
+    __syncthreads();
+    if (q0 + g < Q) {  // group g adds up quantity q0 + g
+      double t = buf[0][g][x];
+#pragma unroll
+      for (int j = 1; j < kGroups; ++j) t += buf[j][g][x];
+      fin[q0 + g][x] = t;
+    }
+    __syncthreads();
+  }
+}
+
+// unit vector of the angles, as the reference forms it: FP32 sines and cosines, FP64 products
+__device__ __forceinline__ void direction(float th, float ph, double (&x)[3]) {
+  float st, ct, sp, cp;
+  sincosf(th, &st, &ct);
+  sincosf(ph, &sp, &cp);
+  x[0] = (double)st * cp;
+  x[1] = (double)st * sp;
+  x[2] = (double)ct;
+}
+
+// adds x x^T to the upper triangle t = {xx, xy, xz, yy, yz, zz}
+__device__ __forceinline__ void add_dyad(double* t, const double (&x)[3]) {
+  t[0] += x[0] * x[0];
+  t[1] += x[0] * x[1];
+  t[2] += x[0] * x[2];
+  t[3] += x[1] * x[1];
+  t[4] += x[1] * x[2];
+  t[5] += x[2] * x[2];
+}
+
+__device__ __forceinline__ void full_tensor(double (*t)[kVox], int x, double scale, double (&A)[3][3]) {
+  A[0][0] = t[0][x] * scale;
+  A[0][1] = A[1][0] = t[1][x] * scale;
+  A[0][2] = A[2][0] = t[2][x] * scale;
+  A[1][1] = t[3][x] * scale;
+  A[1][2] = A[2][1] = t[4][x] * scale;
+  A[2][2] = t[5][x] * scale;
+}
+
 template <int K>
-__device__ void finish_voxel(const FinishArgs& a, int v) {
+__global__ void __launch_bounds__(kVox * kGroups, 3) finish_kernel(FinishArgs a) {
+  constexpr int Q = 6 + 6 * K;
+  __shared__ double sumf[K][kVox], fin[Q][kVox];
+  const int x = threadIdx.x, g = threadIdx.y;
   const int ns = a.nsamples, nvox = a.nvox;
+  const int v = blockIdx.x * kVox + x;
+  const bool in = v < nvox;
   const size_t row = (size_t)ns * nvox;
-  const float* rec = a.records + v;
+  const float* rec = a.records + (in ? v : 0);
   // the fibre order first, from the sums of f over the samples (the f rows, a fifth of the
   // records): sort (sum f, index) ascending and read it backwards (CUDA/samples.cu:299-330)
-  double sumf[K];
+  {
+    double sf[K];
 #pragma unroll
-  for (int k = 0; k < K; ++k) sumf[k] = 0;
-  for (int s = 0; s < ns; ++s) {
+    for (int k = 0; k < K; ++k) sf[k] = 0;
+    if (in)
+      for (int s = g; s < ns; s += kGroups)
 #pragma unroll
-    for (int k = 0; k < K; ++k) sumf[k] += rec[(8 + 3 * k) * row + (size_t)s * nvox];
+        for (int k = 0; k < K; ++k) sf[k] += __ldg(rec + (8 + 3 * k) * row + (size_t)s * nvox);
+    sum_groups<K>(sf, sumf);
   }
   int slot[K];  // output position of fibre k: the number of fibres that come before it
 #pragma unroll
@@ -84,138 +149,128 @@ __device__ void finish_voxel(const FinishArgs& a, int v) {
     int rank = 0;
 #pragma unroll
     for (int j = 0; j < K; ++j)
-      if (j != i && (sumf[j] > sumf[i] || (sumf[j] == sumf[i] && j > i))) ++rank;
+      if (j != i && (sumf[j][x] > sumf[i][x] || (sumf[j][x] == sumf[i][x] && j > i))) ++rank;
     slot[i] = rank;
   }
   // one pass over the records: sums, dyadic tensors, and every sample copied to its sorted slot
-  // (each output row is written once, whole sectors at a time across the warp)
-  double sums[6] = {0, 0, 0, 0, 0, 0}, dy[K][3][3];
-#pragma unroll
-  for (int k = 0; k < K; ++k)
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) dy[k][i][j] = 0;
+  // (each output row is written once, a whole line at a time)
   const bpx_outputs& out = a.out;
-  for (int s = 0; s < ns; ++s) {
-    const size_t o = (size_t)s * nvox;
+  double val[Q];
 #pragma unroll
-    for (int r = 0; r < 6; ++r) sums[r] += rec[r * row + o];
+  for (int q = 0; q < Q; ++q) val[q] = 0;
+  if (in) {
+    for (int s = g; s < ns; s += kGroups) {
+      const size_t o = (size_t)s * nvox;
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const float th = rec[(6 + 3 * k) * row + o], ph = rec[(7 + 3 * k) * row + o];
-      float st, ct, sp, cp;
-      sincosf(th, &st, &ct);
-      sincosf(ph, &sp, &cp);
-      const double x[3] = {(double)st * cp, (double)st * sp, (double)ct};
+      for (int r = 0; r < 6; ++r) val[r] += __ldg(rec + r * row + o);
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) dy[k][i][j] += x[i] * x[j];
-      const size_t oo = ((size_t)slot[k] * ns + s) * nvox + v;
-      if (out.th) out.th[oo] = th;
-      if (out.ph) out.ph[oo] = ph;
-      if (out.f) out.f[oo] = rec[(8 + 3 * k) * row + o];
+      for (int k = 0; k < K; ++k) {
+        const float th = __ldg(rec + (6 + 3 * k) * row + o), ph = __ldg(rec + (7 + 3 * k) * row + o);
+        const size_t oo = ((size_t)slot[k] * ns + s) * nvox + v;
+        if (out.th) out.th[oo] = th;
+        if (out.ph) out.ph[oo] = ph;
+        if (out.f) out.f[oo] = __ldg(rec + (8 + 3 * k) * row + o);
+        double d[3];
+        direction(th, ph, d);
+        add_dyad(val + 6 + 6 * k, d);
+      }
     }
   }
+  sum_groups<Q>(val, fin);
+  if (!in) return;
   const double inv = 1.0 / ns;
-  if (out.mean_d) out.mean_d[v] = (float)(sums[0] * inv);
-  if (out.mean_f0) out.mean_f0[v] = (float)(sums[1] * inv);
-  if (out.mean_tau) out.mean_tau[v] = (float)(sums[2] * inv);
-  if (out.mean_dstd) out.mean_dstd[v] = (float)(sums[3] * inv);
-  if (out.mean_R) out.mean_R[v] = (float)(sums[4] * inv);
-  if (out.mean_S0) out.mean_S0[v] = (float)(sums[5] * inv);
+  if (g < K) {  // warp g: fibre g's mean and dyad, to its sorted slot
+    int o = 0;
 #pragma unroll
-  for (int o = 0; o < K; ++o) {
-    int src = 0;
-#pragma unroll
-    for (int i = 0; i < K; ++i)
-      if (slot[i] == o) src = i;
-    double sf = 0, A[3][3];
-#pragma unroll
-    for (int i = 0; i < K; ++i)
-      if (i == src) {
-        sf = sumf[i];
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) A[r][c] = dy[i][r][c];
-      }
-    if (out.mean_f) out.mean_f[(size_t)o * nvox + v] = (float)(sf * inv);
+    for (int k = 0; k < K; ++k)
+      if (k == g) o = slot[k];
+    if (out.mean_f) out.mean_f[(size_t)o * nvox + v] = (float)(sumf[g][x] * inv);
     if (out.dyads) {
-      double pv[3];
+      double A[3][3], pv[3];
+      full_tensor(fin + 6 + 6 * g, x, 1.0, A);
       principal_vector(A, pv);
 #pragma unroll
       for (int r = 0; r < 3; ++r) out.dyads[((size_t)o * 3 + r) * nvox + v] = (float)pv[r];
     }
+  } else if (g == kGroups - 1) {
+    float* mean[6] = {out.mean_d, out.mean_f0, out.mean_tau, out.mean_dstd, out.mean_R, out.mean_S0};
+#pragma unroll
+    for (int r = 0; r < 6; ++r)
+      if (mean[r]) mean[r][v] = (float)(fin[r][x] * inv);
   }
 }
 
-// One thread per voxel (grid-stride).  The f rows are read first to fix the fibre order, then
-// every record once more while the sums are formed and the samples copied to their sorted slots.
-template <int K>
-__global__ void finish_kernel(FinishArgs a) {
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < a.nvox; v += gridDim.x * blockDim.x) finish_voxel<K>(a, v);
-}
-
 // bedpostx_postproc_gpu.sh arithmetic (CUDA/bedpostx_postproc_gpu.sh:20-49) on the finished
-// outputs, one thread per voxel: fslmaths -Tmean of merged_th/ph, the dispersion of each fibre's
+// outputs, in the layout of finish_kernel: fslmaths -Tmean of merged_th/ph, the dispersion of each fibre's
 // mean dyadic tensor (make_dyadic_vectors.cc:60-92: 1 - max |eigenvalue|), maskdyads
 // (dyads{k} where mean_f{k} >= thr, fslmaths -thr -bin -mul), the _modf{k} scaling by
 // mean_f{k}/mean_f1 (fslmaths -div gives 0 where the divisor is 0) and mean_fsumsamples.
 template <int K>
-__global__ void postproc_kernel(PostArgs a) {
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= a.nvox) return;
+__global__ void __launch_bounds__(kVox * kGroups, 3) postproc_kernel(PostArgs a) {
+  constexpr int Q = 8 * K;  // per fibre: sum th, sum ph, the tensor's upper triangle
+  __shared__ double fin[Q][kVox];
+  const int x = threadIdx.x, g = threadIdx.y;
   const int ns = a.nsamples, nvox = a.nvox;
+  const int v = blockIdx.x * kVox + x;
+  const bool in = v < nvox;
   const bpx_postproc& p = a.post;
-  float mf[K];
-  double fsum = 0.0;
+  double val[Q];
 #pragma unroll
-  for (int k = 0; k < K; ++k) {
-    mf[k] = a.mean_f[(size_t)k * nvox + v];
-    fsum += mf[k];
-    double sth = 0, sph = 0, A[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    for (int s = 0; s < ns; ++s) {
-      const size_t o = ((size_t)k * ns + s) * nvox + v;
-      const float th = a.th[o], ph = a.ph[o];
-      sth += th;
-      sph += ph;
-      float st, ct, sp, cp;
-      sincosf(th, &st, &ct);
-      sincosf(ph, &sp, &cp);
-      const double x[3] = {(double)st * cp, (double)st * sp, (double)ct};
+  for (int q = 0; q < Q; ++q) val[q] = 0;
+  if (in) {
+    for (int s = g; s < ns; s += kGroups) {
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) A[i][j] += x[i] * x[j] / ns;
-    }
-    if (p.mean_th) p.mean_th[(size_t)k * nvox + v] = (float)(sth / ns);
-    if (p.mean_ph) p.mean_ph[(size_t)k * nvox + v] = (float)(sph / ns);
-    if (p.dispersion) {
-      double pv[3];
-      const double lmax = principal_vector(A, pv);  // the tensor is positive semi-definite
-      p.dispersion[(size_t)k * nvox + v] = (float)(1.0 - fabs(lmax));
+      for (int k = 0; k < K; ++k) {
+        const size_t o = ((size_t)k * ns + s) * nvox + v;
+        const float th = __ldg(a.th + o), ph = __ldg(a.ph + o);
+        val[8 * k] += th;
+        val[8 * k + 1] += ph;
+        double d[3];
+        direction(th, ph, d);
+        add_dyad(val + 8 * k + 2, d);
+      }
     }
   }
-  if (p.mean_fsum) p.mean_fsum[v] = (float)fsum;
+  sum_groups<Q>(val, fin);
+  if (!in) return;
+  if (g < K) {
+    const size_t o = (size_t)g * nvox + v;
+    if (p.mean_th) p.mean_th[o] = (float)(fin[8 * g][x] / ns);
+    if (p.mean_ph) p.mean_ph[o] = (float)(fin[8 * g + 1][x] / ns);
+    if (p.dispersion) {
+      double A[3][3], pv[3];
+      full_tensor(fin + 8 * g + 2, x, 1.0 / ns, A);
+      const double lmax = principal_vector(A, pv);  // the tensor is positive semi-definite
+      p.dispersion[o] = (float)(1.0 - fabs(lmax));
+    }
+  } else if (g == kGroups - 1) {
+    float mf[K];
+    double fsum = 0.0;
 #pragma unroll
-  for (int k = 1; k < K; ++k) {
-    const bool keep = mf[k] >= a.thr && mf[k] != 0.f;
-    const float ratio = mf[0] != 0.f ? mf[k] / mf[0] : 0.f;
+    for (int k = 0; k < K; ++k) {
+      mf[k] = a.mean_f[(size_t)k * nvox + v];
+      fsum += mf[k];
+    }
+    if (p.mean_fsum) p.mean_fsum[v] = (float)fsum;
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      const size_t o = ((size_t)k * 3 + r) * nvox + v;
-      const float dt = keep ? a.dyads[o] : 0.f;
-      if (p.dyads_thr) p.dyads_thr[o] = dt;
-      if (p.dyads_modf) p.dyads_modf[o] = dt * ratio;
+    for (int k = 1; k < K; ++k) {
+      const bool keep = mf[k] >= a.thr && mf[k] != 0.f;
+      const float ratio = mf[0] != 0.f ? mf[k] / mf[0] : 0.f;
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const size_t o = ((size_t)k * 3 + r) * nvox + v;
+        const float dt = keep ? a.dyads[o] : 0.f;
+        if (p.dyads_thr) p.dyads_thr[o] = dt;
+        if (p.dyads_modf) p.dyads_modf[o] = dt * ratio;
+      }
     }
   }
 }
 
 cudaError_t launch_postproc(const PostArgs& a, cudaStream_t s) {
   if (a.nvox == 0) return cudaSuccess;
-  const int threads = 128, grid = (a.nvox + threads - 1) / threads;
+  const dim3 threads(kVox, kGroups);
+  const int grid = (a.nvox - 1) / kVox + 1;
   switch (a.nfib) {
     case 1: postproc_kernel<1><<<grid, threads, 0, s>>>(a); break;
     case 2: postproc_kernel<2><<<grid, threads, 0, s>>>(a); break;
@@ -227,8 +282,8 @@ cudaError_t launch_postproc(const PostArgs& a, cudaStream_t s) {
 
 cudaError_t launch_finish(const FinishArgs& a, cudaStream_t s) {
   if (a.nvox == 0) return cudaSuccess;
-  const int threads = 128;
-  const int grid = (a.nvox + threads - 1) / threads;
+  const dim3 threads(kVox, kGroups);
+  const int grid = (a.nvox - 1) / kVox + 1;
   switch (a.nfib) {
     case 1: finish_kernel<1><<<grid, threads, 0, s>>>(a); break;
     case 2: finish_kernel<2><<<grid, threads, 0, s>>>(a); break;
