@@ -13,9 +13,17 @@
 //   K-major tile  [K/8 groups][rows][8]  -> LBO (K direction) = rows*16 B, SBO (rows) = 128 B
 //   MN-major tile [MN/8 groups][K][8]    -> LBO (K direction) = 128 B,    SBO (MN)   = K*16 B
 // One thread issues TMA and MMA (M = 128, N = tile width <= 256, K = 16 per instruction) through
-// a two-stage mbarrier ring; four warps then read their 32 TMEM lanes each (tcgen05.ld) and run
-// the epilogue.  Every mbarrier wait is bounded (about a second), after which the kernel records
-// an error code, waits (bounded) for its own MMAs and releases its tensor memory.
+// an mbarrier ring of two to four stages; eight warps then read the accumulator (tcgen05.ld: warp w
+// the 32 TMEM lanes w%4, every second block of 32 columns) and run the epilogue.  Every mbarrier
+// wait is bounded (about a second), after which the kernel records an error code, waits (bounded) for
+// its own MMAs and releases its tensor memory.
+//
+// The network's contractions are 2 to 5 chunks deep, so a CTA's time is its epilogue (256 erff per row
+// of a 256-wide tile): bound by FP32 issue with too few warps, not by the tensor pipe.  Hence eight
+// epilogue warps and two CTAs per SM, a tile width chosen so that the CTAs fill the device
+// (choose_ntile), and for the weight gradients, whose output is a few tiles but whose contraction is
+// the whole batch, a split of the contraction over CTAs (GemmArgs::split; the partial sums are added
+// in split order by the caller's reduction, so a run reproduces) with all layers in one launch.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -32,16 +40,17 @@ namespace gemm {
 
 constexpr int kTileM = 128;
 constexpr int kChunkK = 64;
-constexpr int kThreads = 128;
+constexpr int kThreads = 256;
+constexpr int kMaxStages = 4;
 constexpr long long kWaitCycles = 2000000000ll;  // ~1 s at 2 GHz
-// epilogue staging per warp: a 32 x 32 fp32 block (rows padded to 36 floats) and a 32 x 32 bf16
-// block (rows padded to 80 bytes); both pitches keep 16-byte alignment and spread a quarter-warp's
-// 16-byte accesses over distinct banks
+// epilogue staging per warp: a 32 x 32 fp32 block (rows padded to 36 floats) or, in the same place, a
+// 32 x 32 bf16 block (rows padded to 80 bytes); both pitches keep 16-byte alignment and spread a
+// quarter-warp's 16-byte accesses over distinct banks
 constexpr int kPitchF = 36;
 constexpr int kPitchB = 80;
-constexpr int kEpiWarpBytes = 32 * kPitchF * 4 + 32 * kPitchB;
-static_assert((kThreads / 32) * kEpiWarpBytes <= 2 * kTileM * kChunkK * 2, "epilogue tiles must fit the A stages");
-static_assert(kEpiWarpBytes % 16 == 0 && (32 * kPitchF * 4) % 16 == 0, "epilogue tiles must stay 16-byte aligned");
+constexpr int kEpiWarpBytes = 32 * kPitchF * 4;
+static_assert((kThreads / 32) * kEpiWarpBytes <= 2 * (kTileM + 32) * kChunkK * 2, "epilogue tiles must fit two stages");
+static_assert(kEpiWarpBytes % 16 == 0 && 32 * kPitchB <= kEpiWarpBytes, "the bf16 block shares the fp32 block's place");
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -113,27 +122,49 @@ __device__ __forceinline__ uint16_t to_bf16(float x) {
 
 struct Smem {
   float bias[256];  // the tile's bias columns, staged once for the epilogue (16-byte aligned)
-  uint64_t full[2], empty[2], done;
+  uint64_t full[kMaxStages], empty[kMaxStages], done;
   uint32_t tmem_base;
 };
 
-__global__ void __launch_bounds__(kThreads, 1)
-    gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, GemmArgs g) {
+// the problems of a launch; problem p has CTAs first[p] .. first[p+1]-1, its tiles along M fastest, then
+// along N, then the splits
+struct Batch {
+  CUtensorMap a[kMaxProblems], b[kMaxProblems];
+  GemmArgs g[kMaxProblems];
+  int first[kMaxProblems + 1];
+  int n, stages;
+};
+
+__host__ __device__ inline int tiles_m(const GemmArgs& g) { return (g.M + kTileM - 1) / kTileM; }
+__host__ __device__ inline int tiles_n(const GemmArgs& g) { return (g.N + g.ntile - 1) / g.ntile; }
+
+__global__ void __launch_bounds__(kThreads, 2) gemm_kernel(const __grid_constant__ Batch batch) {
   extern __shared__ __align__(1024) unsigned char dsmem[];
+  int prob = 0;
+  while (prob + 1 < batch.n && (int)blockIdx.x >= batch.first[prob + 1]) ++prob;
+  const GemmArgs& g = batch.g[prob];
+  const CUtensorMap &map_a = batch.a[prob], &map_b = batch.b[prob];
+  const int stages = batch.stages;
+  const int tile = blockIdx.x - batch.first[prob];
+  const int tm = tiles_m(g), tn = tiles_n(g);
+  const int bx = tile % tm, by = tile / tm % tn, bz = tile / (tm * tn);
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(dsmem) + 1023) & ~uintptr_t(1023));
   const int nt = g.ntile;
   const uint32_t a_bytes = kTileM * kChunkK * 2, b_bytes = (uint32_t)nt * kChunkK * 2;
   const uint32_t stage_bytes = a_bytes + b_bytes;
-  Smem* sm = reinterpret_cast<Smem*>(base + 2 * stage_bytes);
+  Smem* sm = reinterpret_cast<Smem*>(base + stages * stage_bytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * kTileM, n0 = blockIdx.y * nt;
+  const int m0 = bx * kTileM, n0 = by * nt;
+  // this CTA's chunks of the contraction: [kc0, kc1)
+  const int nk = (g.K + kChunkK - 1) / kChunkK, nsplit = g.split > 1 ? g.split : 1;
+  const int kc0 = (int)((long long)nk * bz / nsplit), kc1 = (int)((long long)nk * (bz + 1) / nsplit);
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" : : "r"(smem_u32(&sm->tmem_base)), "r"(nt));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (threadIdx.x == 0) {
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < stages; ++s) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" : : "r"(smem_u32(&sm->full[s])));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" : : "r"(smem_u32(&sm->empty[s])));
     }
@@ -146,11 +177,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tmem = sm->tmem_base;
 
   if (threadIdx.x == 0) {
-    const int nk = (g.K + kChunkK - 1) / kChunkK;
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)g.a_mn << 15) | ((uint32_t)g.b_mn << 16) |
                            ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
-    auto load = [&](int kc) {
-      const int s = kc & 1;
+    auto load = [&](int kc, int s) {
       const uint32_t sa = smem_u32(base + s * stage_bytes), sb = sa + a_bytes;
       const uint32_t bar = smem_u32(&sm->full[s]);
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" : : "r"(bar), "r"(stage_bytes) : "memory");
@@ -164,10 +193,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         tma_load_3d(sb, &map_b, 0, n0, kc * (kChunkK / 8), bar);
     };
     bool ok = true;
-    for (int kc = 0; kc < 2 && kc < nk; ++kc) load(kc);
-    for (int kc = 0; kc < nk && ok; ++kc) {
-      const int s = kc & 1;
-      const uint32_t ph = (kc >> 1) & 1;
+    for (int i = 0; i < stages && kc0 + i < kc1; ++i) load(kc0 + i, i);
+    int s = 0;
+    uint32_t ph = 0;
+    for (int kc = kc0; kc < kc1; ++kc) {
       if (!mbar_wait(smem_u32(&sm->full[s]), ph)) {
         ok = false;
         break;
@@ -180,15 +209,19 @@ __global__ void __launch_bounds__(kThreads, 1)
                                    : smem_desc(sa + ks * 2 * kTileM * 16, kTileM * 16, 128);
         const uint64_t db = g.b_mn ? smem_desc(sb + ks * 256, 128, kChunkK * 16)
                                    : smem_desc(sb + ks * 2 * nt * 16, nt * 16, 128);
-        mma_bf16(tmem, da, db, idesc, (kc | ks) != 0);
+        mma_bf16(tmem, da, db, idesc, (kc != kc0) || ks != 0);
       }
       mma_commit(smem_u32(&sm->empty[s]));
-      if (kc + 2 < nk) {
+      if (kc + stages < kc1) {
         if (!mbar_wait(smem_u32(&sm->empty[s]), ph)) {
           ok = false;
           break;
         }
-        load(kc + 2);
+        load(kc + stages, s);
+      }
+      if (++s == stages) {
+        s = 0;
+        ph ^= 1;
       }
     }
     if (!ok && g.error) atomicExch(g.error, 1);
@@ -205,7 +238,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
-  // epilogue: warp w owns accumulator rows 32w..32w+31 (TMEM lanes), 32 columns at a time.  A lane
+  // epilogue: warp w owns accumulator rows 32(w%4) .. +31 (its TMEM lanes) of every second block of 32
+  // columns.  A lane
   // holds one row of a 32x32 block, so it is turned around through a per-warp shared-memory tile:
   // lanes write their rows, then read the block back so that consecutive lanes cover consecutive
   // columns of a row, and the global stores (and the GELU-derivative's loads of z) are whole
@@ -213,9 +247,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   // idle once every MMA has completed (the done barrier above).
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   float* tf = reinterpret_cast<float*>(base + warp * kEpiWarpBytes);  // [32][kPitchF] fp32 block
-  unsigned char* tb = base + warp * kEpiWarpBytes + 32 * kPitchF * 4;  // [32][kPitchB] bytes, bf16 block
+  unsigned char* tb = base + warp * kEpiWarpBytes;  // [32][kPitchB] bytes, bf16 block (the same place)
   const bool all_done = __all_sync(0xffffffffu, done);
-  const int row0 = m0 + 32 * warp;
+  const int quad = warp & 3, half = warp >> 2;
+  const int row0 = m0 + 32 * quad;
   auto aligned16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   // the block's 32 rows x 32 fp32 columns, lane = row, to out (row-major, leading dimension ld)
   auto put_f32 = [&](const float (&v)[32], float* out, int ld, int col0) {
@@ -295,10 +330,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     __syncwarp();
   };
-  for (int c = 0; c < nt / 32; ++c) {
+  float* out_f32 = g.out_f32 ? g.out_f32 + (size_t)bz * g.split_stride : nullptr;
+  for (int c = half; c < nt / 32; c += 2) {
     float v[32];
     __syncwarp();
-    tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(c * 32), v);
+    tmem_ld32(tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)(c * 32), v);
     const int col0 = n0 + c * 32;
     if (!all_done || row0 >= g.M || col0 >= g.N) continue;  // warp-uniform
     const float4* sb4 = reinterpret_cast<const float4*>(sm->bias + c * 32);
@@ -313,9 +349,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
     if (g.epi == kEpiStoreF32 || g.epi == kEpiBias) {
-      put_f32(v, g.out_f32, g.ld_out, col0);
+      put_f32(v, out_f32, g.ld_out, col0);
     } else if (g.epi == kEpiBiasGelu) {
-      if (g.out_f32) put_f32(v, g.out_f32, g.ld_out, col0);
+      if (out_f32) put_f32(v, out_f32, g.ld_out, col0);
       uint32_t h[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j)
@@ -375,13 +411,27 @@ static bool make_map(CUtensorMap* m, const uint16_t* ptr, int rows, int cols, in
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-size_t smem_bytes(int ntile) { return 2 * (size_t)(kTileM * kChunkK * 2 + ntile * kChunkK * 2) + 1024 + sizeof(Smem) + 64; }
+size_t smem_bytes(int ntile, int stages) {
+  return stages * (size_t)(kTileM * kChunkK * 2 + ntile * kChunkK * 2) + 1024 + sizeof(Smem) + 64;
+}
 
-// The kernel's dynamic shared-memory limit is raised once per device to what the widest tile
-// (256 columns) needs, and never lowered: a launch with a narrower tile needs less, and a CUDA graph
-// whose nodes were captured with different tile widths stays launchable whatever was set last.
-// (Setting the limit per launch to that launch's own need left it at the last layer's 42 KB after a
-// forward pass, below the 99 KB of the hidden layers' nodes.)
+// Stages of the ring: as many as keep two CTAs on an SM (about 100 KB each) and the contraction can
+// use; a wider tile's stage is larger, so 256 columns get two, 64 columns four.
+int choose_stages(int ntile, int chunks) {
+  const int fit = ntile >= 256 ? 2 : ntile >= 128 ? 3 : kMaxStages;
+  return chunks < 2 ? 2 : chunks < fit ? chunks : fit;
+}
+
+int choose_ntile(int M, int N) {
+  int nt = N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : 256;
+  const long long tm = (M + kTileM - 1) / kTileM;
+  while (nt > 64 && tm * ((N + nt - 1) / nt) < sm_count()) nt /= 2;
+  return nt;
+}
+
+// The kernel's dynamic shared-memory limit is raised once per device to what the largest ring
+// needs, and never lowered: a launch with a smaller one needs less, and a CUDA graph whose nodes were
+// captured with different tile widths stays launchable whatever was set last.
 constexpr int kMaxDevices = 64;
 cudaError_t set_smem_limit_once() {
   static std::mutex mu;
@@ -393,7 +443,10 @@ cudaError_t set_smem_limit_once() {
   std::lock_guard<std::mutex> lk(mu);
   const uint64_t ctx = context_id();
   if (ctx != 0 && done_ctx[dev] == ctx) return cudaSuccess;
-  e = cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(256));
+  size_t most = smem_bytes(256, 2);
+  if (smem_bytes(128, 3) > most) most = smem_bytes(128, 3);
+  if (smem_bytes(64, kMaxStages) > most) most = smem_bytes(64, kMaxStages);
+  e = cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
   if (e == cudaSuccess) done_ctx[dev] = context_id();
   return e;
 }
@@ -406,26 +459,48 @@ const char* check(const GemmOperands& op, const GemmArgs& g) {
   // contiguous extents must be whole groups of 8 elements
   if ((g.a_mn ? g.M : g.K) % 8 || (g.b_mn ? g.N : g.K) % 8) return "GEMM contiguous extents must be multiples of 8";
   if (g.M > (1 << 24) || g.N > (1 << 24) || g.K > (1 << 24)) return "GEMM too large";
+  if (g.split > (g.K + kChunkK - 1) / kChunkK) return "GEMM split into more parts than the contraction has chunks";
   return nullptr;
 }
 
-cudaError_t launch(const GemmOperands& op, const GemmArgs& g, cudaStream_t s, const char** why) {
-  *why = check(op, g);
-  if (*why) return cudaErrorInvalidValue;
-  CUtensorMap ma, mb;
-  const bool ok_a = g.a_mn ? make_map(&ma, op.a, g.K, g.M, op.lda, kChunkK, kTileM / 8)
-                           : make_map(&ma, op.a, g.M, g.K, op.lda, kTileM, kChunkK / 8);
-  const bool ok_b = g.b_mn ? make_map(&mb, op.b, g.K, g.N, op.ldb, kChunkK, g.ntile / 8)
-                           : make_map(&mb, op.b, g.N, g.K, op.ldb, g.ntile, kChunkK / 8);
-  if (!ok_a || !ok_b) {
-    *why = "cuTensorMapEncodeTiled failed (driver entry point missing or unsupported tensor shape)";
+cudaError_t launch(const GemmOperands* op, const GemmArgs* g, int problems, cudaStream_t s, const char** why) {
+  *why = nullptr;
+  if (problems < 1 || problems > kMaxProblems) {
+    *why = "GEMM problem count out of range";
     return cudaErrorInvalidValue;
   }
-  const size_t sm = smem_bytes(g.ntile);
+  Batch b;
+  long long blocks = 0;
+  int chunks = 0, nt = 0;
+  for (int i = 0; i < problems; ++i) {
+    *why = check(op[i], g[i]);
+    if (*why) return cudaErrorInvalidValue;
+    const bool ok_a = g[i].a_mn ? make_map(&b.a[i], op[i].a, g[i].K, g[i].M, op[i].lda, kChunkK, kTileM / 8)
+                                : make_map(&b.a[i], op[i].a, g[i].M, g[i].K, op[i].lda, kTileM, kChunkK / 8);
+    const bool ok_b = g[i].b_mn ? make_map(&b.b[i], op[i].b, g[i].K, g[i].N, op[i].ldb, kChunkK, g[i].ntile / 8)
+                                : make_map(&b.b[i], op[i].b, g[i].N, g[i].K, op[i].ldb, g[i].ntile, kChunkK / 8);
+    if (!ok_a || !ok_b) {
+      *why = "cuTensorMapEncodeTiled failed (driver entry point missing or unsupported tensor shape)";
+      return cudaErrorInvalidValue;
+    }
+    b.g[i] = g[i];
+    b.first[i] = (int)blocks;
+    const int split = g[i].split > 1 ? g[i].split : 1;
+    blocks += (long long)tiles_m(g[i]) * tiles_n(g[i]) * split;
+    if (blocks > (1ll << 30)) {
+      *why = "GEMM too large";
+      return cudaErrorInvalidValue;
+    }
+    const int nk = ((g[i].K + kChunkK - 1) / kChunkK + split - 1) / split;
+    if (nk > chunks) chunks = nk;
+    if (g[i].ntile > nt) nt = g[i].ntile;
+  }
+  b.first[problems] = (int)blocks;
+  b.n = problems;
+  b.stages = choose_stages(nt, chunks);
   const cudaError_t attr = set_smem_limit_once();
   if (attr != cudaSuccess) return attr;
-  const dim3 grid((g.M + kTileM - 1) / kTileM, (g.N + g.ntile - 1) / g.ntile);
-  gemm_kernel<<<grid, kThreads, sm, s>>>(ma, mb, g);
+  gemm_kernel<<<(unsigned)blocks, kThreads, smem_bytes(nt, b.stages), s>>>(b);
   return cudaGetLastError();
 }
 

@@ -23,6 +23,8 @@ struct GemmOperands {
 struct GemmArgs {
   int M, N, K;
   int ntile;       // output columns per CTA: 32, 64, 128 or 256
+  int split;       // CTAs that share a tile's contraction (0 or 1: one); split s writes out_f32 + s * split_stride
+  size_t split_stride;
   int a_mn, b_mn;  // operand orientation: 0 = K-major, 1 = MN-major
   int epi;
   float* out_f32;
@@ -35,8 +37,14 @@ struct GemmArgs {
   int* error;  // set to nonzero when a bounded wait gave up
 };
 
+// Problems of one launch (their CTAs run side by side; no problem may read another's output).
+constexpr int kMaxProblems = 5;
+
+// The widest tile whose CTAs fill the device (at least 64 columns, 32 where N is no wider).
+int choose_ntile(int M, int N);
+
 // Validates the arguments (why = reason on failure) and launches on stream s.
-cudaError_t launch(const GemmOperands& op, const GemmArgs& g, cudaStream_t s, const char** why);
+cudaError_t launch(const GemmOperands* op, const GemmArgs* g, int problems, cudaStream_t s, const char** why);
 
 }  // namespace gemm
 }  // namespace bpx

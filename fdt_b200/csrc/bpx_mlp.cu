@@ -74,8 +74,11 @@ struct WeightMap {
   size_t woff[kLayers], wbf[kLayers + 1];
 };
 
-__global__ void cast_weights_kernel(const float* __restrict__ params, WeightMap m, uint16_t* __restrict__ wbf) {
+// BF16 copy of the weights; also clears *zero (the loss a training step accumulates) when given.
+__global__ void cast_weights_kernel(const float* __restrict__ params, WeightMap m, uint16_t* __restrict__ wbf,
+                                    float* __restrict__ zero) {
   const size_t total = m.wbf[kLayers];
+  if (zero && blockIdx.x == 0 && threadIdx.x == 0) *zero = 0.f;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     int l = 0;
 #pragma unroll
@@ -123,67 +126,103 @@ __global__ void features_kernel(int nvox, int ndir, int nin, const float* __rest
 // Loss of one voxel and its gradient with respect to the outputs (averaged over the batch):
 //   sum_j w_j (o_j - t_j)^2 over the scalar outputs, plus, for fibre k, w_{3+3k} times the
 //   sign-invariant direction loss |u u^T - v v^T|_F^2 = |u|^4 - 2 (u.v)^2 + 1 (|v| = 1).
-__global__ void loss_kernel(int batch, const float* __restrict__ out, const float* __restrict__ t,
-                            const float* __restrict__ tw, uint16_t* __restrict__ dz, float* __restrict__ loss) {
+// One warp per row, lane j the output j, so rows are read and written as whole lines (one thread per
+// row took 20.6 us for 4096 rows, this form 5).
+constexpr int kLossRows = 32;  // rows of a block
+__global__ void __launch_bounds__(256) loss_kernel(int batch, const float* __restrict__ out, const float* __restrict__ t,
+                                                   const float* __restrict__ tw, uint16_t* __restrict__ dz,
+                                                   float* __restrict__ loss) {
   __shared__ float red[8];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const float inv_b = 1.f / (float)batch;
+  const bool dir = j >= 3 && j < 12;
+  const int u0 = dir ? 3 + (j - 3) / 3 * 3 : 0;  // first component of this lane's direction
   float L = 0.f;
-  if (i < batch) {
-    const float* o = out + (size_t)i * kOut;
-    const float* tt = t + (size_t)i * kOut;
-    const float* ww = tw + (size_t)i * kOut;
-    float g[kOut];
-    const float inv_b = 1.f / (float)batch;
-#pragma unroll
-    for (int j = 0; j < kOut; ++j) g[j] = 0.f;
-#pragma unroll
-    for (int j = 0; j < kOut; ++j) {
-      if (j >= 3 && j < 12) continue;
-      const float e = o[j] - tt[j];
-      L += ww[j] * e * e;
-      g[j] = 2.f * ww[j] * e * inv_b;
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const float wd = ww[3 + 3 * k];
-      const float ux = o[3 + 3 * k], uy = o[4 + 3 * k], uz = o[5 + 3 * k];
-      const float vx = tt[3 + 3 * k], vy = tt[4 + 3 * k], vz = tt[5 + 3 * k];
+  for (int r = 0; r < kLossRows / 8; ++r) {
+    const int i = blockIdx.x * kLossRows + r * 8 + w;
+    if (i >= batch) break;  // warp-uniform
+    const float o = out[(size_t)i * kOut + j], tt = t[(size_t)i * kOut + j], ww = tw[(size_t)i * kOut + j];
+    const float ux = __shfl_sync(0xffffffffu, o, u0), uy = __shfl_sync(0xffffffffu, o, u0 + 1),
+                uz = __shfl_sync(0xffffffffu, o, u0 + 2);
+    const float vx = __shfl_sync(0xffffffffu, tt, u0), vy = __shfl_sync(0xffffffffu, tt, u0 + 1),
+                vz = __shfl_sync(0xffffffffu, tt, u0 + 2);
+    const float wd = __shfl_sync(0xffffffffu, ww, u0);
+    float g;
+    if (dir) {
       const float uu = ux * ux + uy * uy + uz * uz, uv = ux * vx + uy * vy + uz * vz;
-      L += wd * (uu * uu - 2.f * uv * uv + 1.f);
+      if (j == u0) L += wd * (uu * uu - 2.f * uv * uv + 1.f);
       const float a = 4.f * wd * uu * inv_b, c = -4.f * wd * uv * inv_b;
-      g[3 + 3 * k] = a * ux + c * vx;
-      g[4 + 3 * k] = a * uy + c * vy;
-      g[5 + 3 * k] = a * uz + c * vz;
+      g = a * o + c * tt;
+    } else {
+      const float e = o - tt;
+      L += ww * e * e;
+      g = 2.f * ww * e * inv_b;
     }
-    uint16_t* d = dz + (size_t)i * kOut;
-#pragma unroll
-    for (int j = 0; j < kOut; ++j) d[j] = __bfloat16_as_ushort(__float2bfloat16_rn(g[j]));
+    dz[(size_t)i * kOut + j] = __bfloat16_as_ushort(__float2bfloat16_rn(g));
   }
   L = group_sum<32>(L);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = L;
+  if (j == 0) red[w] = L;
   __syncthreads();
   if (threadIdx.x == 0) {
     float s = 0.f;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
+    for (int q = 0; q < 8; ++q) s += red[q];
     atomicAdd(loss, s / (float)batch);
   }
 }
 
-// db[n] = sum over rows of dz[r][n] (bf16 in, fp32 out); block = 256 threads covers 32 columns.
-__global__ void colsum_kernel(int rows, int cols, const uint16_t* __restrict__ dz, float* __restrict__ db) {
-  __shared__ float red[8][33];
-  const int c = blockIdx.x * 32 + (threadIdx.x & 31);
-  const int r0 = threadIdx.x >> 5;
-  float s = 0.f;
-  if (c < cols)
-    for (int r = r0; r < rows; r += 8) s += __bfloat162float(__ushort_as_bfloat16(dz[(size_t)r * cols + c]));
-  red[r0][threadIdx.x & 31] = s;
-  __syncthreads();
-  if (r0 == 0 && c < cols) {
-    float t = 0.f;
-    for (int j = 0; j < 8; ++j) t += red[j][threadIdx.x & 31];
-    db[c] = t;
+// The gradients from what the backward pass leaves: a weight is the sum of its contraction splits (part:
+// layer l's at splits * wbf[l], [splits][n][k]), a bias the column sum of its layer's dz [batch][n].
+// Blocks below bias_blocks take 32 bias columns each, warp w every eighth row in order; each thread's
+// additions are one chain, so it keeps kBiasAhead loads in flight (a launch per layer with one load at a
+// time took 54 us each).  The other blocks take weights.
+constexpr int kBiasAhead = 32;
+struct GradMap {
+  size_t woff[kLayers], boff[kLayers], wbf[kLayers + 1];
+  const uint16_t* dz[kLayers];
+  int n[kLayers];
+  int splits, batch, bias_blocks;
+};
+__global__ void __launch_bounds__(256) grad_reduce_kernel(GradMap m, const float* __restrict__ part,
+                                                          float* __restrict__ grads) {
+  if ((int)blockIdx.x < m.bias_blocks) {
+    __shared__ float red[8][33];
+    int l = 0, c0 = blockIdx.x * 32;
+    while (c0 >= m.n[l]) c0 -= m.n[l++];
+    const int c = c0 + (threadIdx.x & 31), r0 = threadIdx.x >> 5, n = m.n[l];
+    const uint16_t* col = m.dz[l] + c;
+    float s = 0.f;
+    int r = r0;
+    for (; r + 8 * (kBiasAhead - 1) < m.batch; r += 8 * kBiasAhead) {
+      uint16_t t[kBiasAhead];
+#pragma unroll
+      for (int q = 0; q < kBiasAhead; ++q) t[q] = __ldg(col + (size_t)(r + 8 * q) * n);
+#pragma unroll
+      for (int q = 0; q < kBiasAhead; ++q) s += __bfloat162float(__ushort_as_bfloat16(t[q]));
+    }
+    for (; r < m.batch; r += 8) s += __bfloat162float(__ushort_as_bfloat16(col[(size_t)r * n]));
+    red[r0][threadIdx.x & 31] = s;
+    __syncthreads();
+    if (r0 == 0) {
+      float t = 0.f;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) t += red[q][threadIdx.x & 31];
+      grads[m.boff[l] + c] = t;
+    }
+    return;
   }
+  const size_t total = m.wbf[kLayers];
+  const size_t i = (size_t)(blockIdx.x - m.bias_blocks) * blockDim.x + threadIdx.x;
+  if (i >= total) return;
+  int l = 0;
+#pragma unroll
+  for (int q = 1; q < kLayers; ++q)
+    if (i >= m.wbf[q]) l = q;
+  const size_t e = i - m.wbf[l], stride = m.wbf[l + 1] - m.wbf[l];
+  const float* p = part + (size_t)m.splits * m.wbf[l] + e;
+  float s = 0.f;
+#pragma unroll 4
+  for (int q = 0; q < m.splits; ++q) s += p[(size_t)q * stride];
+  grads[m.woff[l] + e] = s;
 }
 
 __global__ void adam_kernel(size_t n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
@@ -350,6 +389,14 @@ size_t a256(size_t x) { return (x + 255) & ~(size_t)255; }
     if (e_ != cudaSuccess) return api_cuda_fail(e_, #call);     \
   } while (0)
 
+bpx_status launch_gemms(const gemm::GemmOperands* op, const gemm::GemmArgs* g, int n, cudaStream_t s) {
+  const char* why = nullptr;
+  const cudaError_t e = gemm::launch(op, g, n, s, &why);
+  if (why) return api_fail(BPX_ERR_INVALID_ARG, std::string("tcgen05 GEMM: ") + why);
+  if (e != cudaSuccess) return api_cuda_fail(e, "gemm launch");
+  return BPX_OK;
+}
+
 bpx_status run_gemm(const uint16_t* a, int lda, int a_mn, const uint16_t* b, int ldb, int b_mn, int M, int N, int K,
                     int epi, float* out_f32, int ld_out, uint16_t* out_bf16, int ld_bf16, const float* bias,
                     const float* zin, int ld_zin, int* err, cudaStream_t s) {
@@ -358,7 +405,7 @@ bpx_status run_gemm(const uint16_t* a, int lda, int a_mn, const uint16_t* b, int
   g.M = M;
   g.N = N;
   g.K = K;
-  g.ntile = N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : 256;
+  g.ntile = gemm::choose_ntile(M, N);
   g.a_mn = a_mn;
   g.b_mn = b_mn;
   g.epi = epi;
@@ -370,11 +417,7 @@ bpx_status run_gemm(const uint16_t* a, int lda, int a_mn, const uint16_t* b, int
   g.zin = zin;
   g.ld_zin = ld_zin;
   g.error = err;
-  const char* why = nullptr;
-  const cudaError_t e = gemm::launch(op, g, s, &why);
-  if (why) return api_fail(BPX_ERR_INVALID_ARG, std::string("tcgen05 GEMM: ") + why);
-  if (e != cudaSuccess) return api_cuda_fail(e, "gemm launch");
-  return BPX_OK;
+  return launch_gemms(&op, &g, 1, s);
 }
 
 // per-device error word the GEMM's bounded waits write; read by bpx_mlp_poll_error
@@ -397,14 +440,14 @@ bpx_status error_word(int** out) {
   return BPX_OK;
 }
 
-bpx_status cast_weights(const Geom& G, const float* params, uint16_t* wbf, cudaStream_t s) {
+bpx_status cast_weights(const Geom& G, const float* params, uint16_t* wbf, float* zero, cudaStream_t s) {
   WeightMap m;
   for (int l = 0; l < kLayers; ++l) {
     m.woff[l] = G.woff[l];
     m.wbf[l] = G.wbf[l];
   }
   m.wbf[kLayers] = G.nw;
-  cast_weights_kernel<<<(unsigned)std::min<size_t>((G.nw + 255) / 256, 4096), 256, 0, s>>>(params, m, wbf);
+  cast_weights_kernel<<<(unsigned)std::min<size_t>((G.nw + 255) / 256, 4096), 256, 0, s>>>(params, m, wbf, zero);
   MLP_CUDA(cudaGetLastError());
   return BPX_OK;
 }
@@ -450,7 +493,7 @@ bpx_status mlp_forward_buffers(int ndir, const float* params, int nvox, const ui
   const Geom G = geom(ndir);
   int* err = nullptr;
   bpx_status st = error_word(&err);
-  if (st == BPX_OK) st = cast_weights(G, params, wbf, s);
+  if (st == BPX_OK) st = cast_weights(G, params, wbf, nullptr, s);
   for (int r0 = 0; st == BPX_OK && r0 < nvox; r0 += chunk_rows) {
     const int n = std::min(chunk_rows, nvox - r0);
     st = forward(G, params, wbf, n, x + (size_t)r0 * G.nin, out + (size_t)r0 * kOut, buf0, buf1, nullptr, nullptr, err,
@@ -528,7 +571,7 @@ bpx_status bpx_mlp_forward_dev(int32_t ndir, const float* params, int32_t nvox, 
   uint16_t* buf0 = (uint16_t*)(p + b_w);
   uint16_t* buf1 = (uint16_t*)(p + b_w + b_act);
   cudaStream_t s = (cudaStream_t)stream;
-  st = cast_weights(G, params, wbf, s);
+  st = cast_weights(G, params, wbf, nullptr, s);
   if (st != BPX_OK) return st;
   for (int r0 = 0; r0 < nvox; r0 += chunk) {
     const int n = std::min(chunk, nvox - r0);
@@ -549,8 +592,15 @@ bpx_status bpx_mlp_train_step_dev(int32_t ndir, const float* params, float* grad
   const size_t B = (size_t)batch;
   const size_t b_w = a256(G.nw * 2), b_a = a256(B * kWidth * 2), b_z = a256(B * kWidth * 4);
   const size_t b_out = a256(B * kOut * 4), b_dz5 = a256(B * kOut * 2);
+  // the weight gradients' outputs are a few tiles each with the whole batch to contract: 32-column
+  // tiles of all layers in one launch, each contraction in two parts, give every SM a CTA at 4096
+  // rows.  (Eight parts are no faster end to end, 165 us a step either way, and move the sums, whose
+  // accumulation the tensor core rounds, nearer to 1e-5 from the undivided ones.)
+  const int chunks = (batch + 63) / 64;
+  const int splits = chunks >= 16 ? 2 : 1;
+  const size_t b_part = a256(G.nw * splits * 4);
   void* ws = nullptr;
-  st = api_workspace(kWsNetwork, b_w + 4 * b_a + 4 * b_z + b_out + b_dz5 + 2 * b_a, &ws);
+  st = api_workspace(kWsNetwork, b_w + 8 * b_a + 4 * b_z + b_out + b_dz5 + b_part, &ws);
   if (st != BPX_OK) return st;
   int* err = nullptr;
   st = error_word(&err);
@@ -558,41 +608,62 @@ bpx_status bpx_mlp_train_step_dev(int32_t ndir, const float* params, float* grad
   char* p = (char*)ws;
   uint16_t* wbf = (uint16_t*)p;
   p += b_w;
-  uint16_t* acts[4];
+  uint16_t *acts[4], *dz[kLayers];
   float* z[4];
   for (int i = 0; i < 4; ++i, p += b_a) acts[i] = (uint16_t*)p;
   for (int i = 0; i < 4; ++i, p += b_z) z[i] = (float*)p;
+  for (int i = 0; i < 4; ++i, p += b_a) dz[i] = (uint16_t*)p;
   float* out = (float*)p;
   p += b_out;
-  uint16_t* dz5 = (uint16_t*)p;
+  dz[kLayers - 1] = (uint16_t*)p;
   p += b_dz5;
-  uint16_t* dzb[2] = {(uint16_t*)p, (uint16_t*)(p + b_a)};
+  float* part = (float*)p;
   cudaStream_t s = (cudaStream_t)stream;
-  st = cast_weights(G, params, wbf, s);
+  st = cast_weights(G, params, wbf, loss, s);
   if (st != BPX_OK) return st;
   st = forward(G, params, wbf, batch, x, out, nullptr, nullptr, z, acts, err, s);
   if (st != BPX_OK) return st;
-  MLP_CUDA(cudaMemsetAsync(loss, 0, sizeof(float), s));
-  loss_kernel<<<(batch + 255) / 256, 256, 0, s>>>(batch, out, targets, tweights, dz5, loss);
+  loss_kernel<<<(batch + kLossRows - 1) / kLossRows, 256, 0, s>>>(batch, out, targets, tweights, dz[kLayers - 1], loss);
   MLP_CUDA(cudaGetLastError());
-  // backward: g = dL/d(layer output); dW_l = g^T a_l, db_l = colsum(g), g <- (g W_l) * gelu'(z_l)
-  const uint16_t* g = dz5;
-  int ldg = kOut;
-  for (int l = kLayers - 1; l >= 0; --l) {
-    const uint16_t* al = l == 0 ? x : acts[l - 1];
-    st = run_gemm(g, ldg, 1, al, G.k[l], 1, G.n[l], G.k[l], batch, gemm::kEpiStoreF32, grads + G.woff[l], G.k[l],
-                  nullptr, 0, nullptr, nullptr, 0, err, s);
+  // backward: dz_l = (dz_{l+1} W_{l+1}) * gelu'(z_l), layer by layer; then every dW_l = dz_l^T a_l in one
+  // launch, and the parts and column sums (db_l) added up
+  for (int l = kLayers - 1; l > 0; --l) {
+    st = run_gemm(dz[l], G.n[l], 0, wbf + G.wbf[l], G.k[l], 1, batch, G.k[l], G.n[l], gemm::kEpiGeluGrad, nullptr, 0,
+                  dz[l - 1], G.k[l], nullptr, z[l - 1], G.k[l], err, s);
     if (st != BPX_OK) return st;
-    colsum_kernel<<<(G.n[l] + 31) / 32, 256, 0, s>>>(batch, G.n[l], g, grads + G.boff[l]);
-    MLP_CUDA(cudaGetLastError());
-    if (l == 0) break;
-    uint16_t* gn = dzb[l & 1];
-    st = run_gemm(g, ldg, 0, wbf + G.wbf[l], G.k[l], 1, batch, G.k[l], G.n[l], gemm::kEpiGeluGrad, nullptr, 0, gn,
-                  G.k[l], nullptr, z[l - 1], G.k[l], err, s);
-    if (st != BPX_OK) return st;
-    g = gn;
-    ldg = G.k[l];
   }
+  static_assert(kLayers <= gemm::kMaxProblems, "one launch holds every layer's weight gradient");
+  gemm::GemmOperands op[kLayers];
+  gemm::GemmArgs g[kLayers];
+  GradMap m;
+  for (int l = 0; l < kLayers; ++l) {
+    op[l] = gemm::GemmOperands{dz[l], l == 0 ? x : acts[l - 1], G.n[l], G.k[l]};
+    g[l] = gemm::GemmArgs{};
+    g[l].M = G.n[l];
+    g[l].N = G.k[l];
+    g[l].K = batch;
+    g[l].ntile = 32;
+    g[l].split = splits;
+    g[l].split_stride = (size_t)G.n[l] * G.k[l];
+    g[l].a_mn = g[l].b_mn = 1;
+    g[l].epi = gemm::kEpiStoreF32;
+    g[l].out_f32 = part + splits * G.wbf[l];
+    g[l].ld_out = G.k[l];
+    g[l].error = err;
+    m.woff[l] = G.woff[l];
+    m.boff[l] = G.boff[l];
+    m.wbf[l] = G.wbf[l];
+    m.n[l] = G.n[l];
+    m.dz[l] = dz[l];
+  }
+  m.wbf[kLayers] = G.nw;
+  m.splits = splits;
+  m.batch = batch;
+  m.bias_blocks = ((kLayers - 1) * kWidth + kOut) / 32;
+  st = launch_gemms(op, g, kLayers, s);
+  if (st != BPX_OK) return st;
+  grad_reduce_kernel<<<(unsigned)(m.bias_blocks + (G.nw + 255) / 256), 256, 0, s>>>(m, part, grads);
+  MLP_CUDA(cudaGetLastError());
   return BPX_OK;
 }
 
