@@ -7,8 +7,10 @@
 // seed, then adds 1 to fdt_paths in every voxel the kept halves passed through (once per voxel:
 // a per-thread open-addressing table of the voxels already counted, entries stamped with the
 // particle so no clearing is needed between particles) and 1 to waytotal.  With an avoid mask,
-// waypoint masks or a distance threshold, the particle's halves are tracked once to learn which
-// are kept, then the kept ones again (the same draws, so the same path) to count them.
+// waypoint masks or a distance threshold, which halves are kept is known only when both have ended:
+// the halves' voxels are listed as they are tracked and the kept lists counted afterwards (with
+// --omatrix2, or targets under a distance threshold, whose counts need the positions or path lengths
+// along the way, the kept halves are tracked again: the same draws, so the same path).
 //
 // The work is a chain of dependent random gathers (the mask at the position and a posterior sample
 // at a randomly rounded position, then the step), so the kernel is latency-bound: a persistent
@@ -21,9 +23,11 @@
 // file is compiled with -fmad=false), sine and cosine from sincos_fast; random numbers from
 // Philox-4x32-10 keyed by the seed, counted by (particle, half, step), eight uniforms per step.
 // The CPU oracle (oracle/track_oracle.c) does the same operations and follows identical paths.
+#include <array>
 #include <cmath>
 #include <cstdint>
 #include <string>
+#include <utility>
 
 #include "bpx.h"
 #include "bpx_device.cuh"
@@ -47,6 +51,8 @@ constexpr int kFeatEuler = 1;  // --modeuler
 constexpr int kFeatLoop = 2;   // --loopcheck
 constexpr int kFeatCount = 4;  // seeds to targets, matrix2, matrix1
 constexpr int kFeatPref = 8;   // --prefdir
+constexpr int kFeatKeep = 16;  // a half's fate waits on its length, the avoid mask or the waypoints
+constexpr int kFeats = 32;
 
 struct TrackArgs {
   bpx_track_options o;
@@ -71,6 +77,10 @@ struct TrackArgs {
   int lcnx, lcny;
   float sx, sy, sz;  // steplength / dx, dy, dz
   float lrx, lry, lrz;  // matrix2: dx / lr_dx, dy / lr_dy, dz / lr_dz
+  // kFeatKeep: per-thread lists [threads][2][list_cap] of the voxels the halves enter, in order (NULL: the
+  // kept halves are tracked a second time to be counted)
+  uint32_t* lists;
+  size_t list_cap;
   uint64_t pid_begin;  // particles [pid_begin, pid_end) of this launch
   uint64_t pid_end;
 };
@@ -274,6 +284,34 @@ struct Tracker {
     return false;  // unreachable: the table holds twice the longest path
   }
 
+  // adds voxel `vox` to fdt_paths (and --omatrix1's row) on the particle's first visit
+  template <int FEAT>
+  __device__ void count_visit(uint32_t vox, int& nvisit, const Counted& cnt) const {
+    if (!first_visit(vox)) return;
+    const int add = a.o.pathdist ? ++nvisit : 1;
+    atomicAdd(paths + vox, add);
+    if ((FEAT & kFeatCount) && a.v.m1_ncols > 0) {
+      // --omatrix1: a seed-mask voxel's fdt_paths count also goes to the seed's row
+      const int c1 = __ldg(a.v.m1_lookup + vox);
+      if (c1 >= 0 && c1 < a.v.m1_ncols) atomicAdd(a.v.matrix1 + (size_t)cnt.seed * a.v.m1_ncols + c1, add);
+    }
+  }
+
+  // counts a kept half from its list of voxels, as half_line counts while it tracks (targets without a
+  // distance threshold: every entry's path is long enough)
+  template <int FEAT>
+  __device__ void count_list(const uint32_t* list, int n, int& nvisit, Counted& cnt) const {
+    for (int i = 0; i < n; ++i) {
+      const uint32_t vox = list[i];
+      count_visit<FEAT>(vox, nvisit, cnt);
+      if ((FEAT & kFeatCount) && a.v.ntargets > 0) {
+        const uint32_t tb = __ldg(a.v.targets + vox) & ~cnt.tflags;
+        for (uint32_t b = tb; b; b &= b - 1) atomicAdd(a.v.seeds_to_targets + (size_t)(__ffs(b) - 1) * a.nseeds + cnt.seed, 1);
+        cnt.tflags |= tb;
+      }
+    }
+  }
+
   // The voxel and posterior sample a step reads (the probabilistic rounding of Tractvolsx::sample):
   // depends only on the position and the step's uniforms, so its loads can be issued together
   // with the mask's.
@@ -370,10 +408,12 @@ struct Tracker {
   // accumulates the waypoint masks passed (over both halves of a particle).  Returns the reject
   // flag: 1 (entered the avoid mask, passed no waypoint, or shorter than distthresh), 2 (passed
   // some waypoints but not all), 0.
-  // FEAT: the feature set compiled in (kFeatEuler, kFeatLoop, kFeatCount)
+  // FEAT: the feature set compiled in (kFeatEuler, kFeatLoop, kFeatCount).  list: the voxels entered
+  // are written there instead (count false), their number to nlist.
   template <int FEAT>
   __device__ int half_line(Particle& P, uint64_t pid, int h, int fibst0, float x0, float y0, float z0,
-                           bool count, uint32_t& flags, int& nvisit, Counted& cnt) {
+                           bool count, uint32_t& flags, int& nvisit, Counted& cnt, uint32_t* list = nullptr,
+                           int* nlist = nullptr) {
     const bpx_track_options& o = a.o;
     const bpx_track_volume& v = a.v;
     bool init_sample = true, avoided = false;
@@ -386,6 +426,7 @@ struct Tracker {
     // a step of steplength mm mostly stays in the voxel of the step before, which is counted
     // already: the visit table is probed only when the voxel changes
     uint32_t last = 0xffffffffu, last_lr = 0xffffffffu;
+    int nl = 0;
     ++lc_stamp;  // every tracked half starts with an empty loopcheck volume
     // --loopcheck: the coarse cell of the step before and the direction stored for it since; the
     // table is read and written only when the cell changes (about every 20 steps of 0.5 mm in 2 mm
@@ -450,17 +491,13 @@ struct Tracker {
         lc_dir = make_float3(P.rx, P.ry, P.rz);
       }
       flags |= way;
+      if ((FEAT & kFeatKeep) && list && vox != last) {
+        last = vox;
+        list[nl++] = vox;  // at most one per step: the list holds nsteps / 2
+      }
       if (count && vox != last) {
         last = vox;
-        if (first_visit(vox)) {
-          const int add = o.pathdist ? ++nvisit : 1;
-          atomicAdd(paths + vox, add);
-          if ((FEAT & kFeatCount) && v.m1_ncols > 0) {
-            // --omatrix1: a seed-mask voxel's fdt_paths count also goes to the seed's row
-            const int c1 = __ldg(v.m1_lookup + vox);
-            if (c1 >= 0 && c1 < v.m1_ncols) atomicAdd(v.matrix1 + (size_t)cnt.seed * v.m1_ncols + c1, add);
-          }
-        }
+        count_visit<FEAT>(vox, nvisit, cnt);
         if ((FEAT & kFeatCount) && v.ntargets > 0) {
           // a target is counted at its first entry on the counted path (a voxel change), if the path
           // is by then at least distthresh long (Counter::update_seedcounts)
@@ -531,6 +568,7 @@ struct Tracker {
         }
       }
     }
+    if ((FEAT & kFeatKeep) && list) *nlist = nl;
     int rej = 0;
     if (v.nwaypoints > 0) {
       const uint32_t all = v.nwaypoints >= 32 ? 0xffffffffu : ((1u << v.nwaypoints) - 1u);
@@ -552,10 +590,7 @@ __global__ void __launch_bounds__(kTrackThreads, kTrackBlocksPerSm) track_kernel
     T.lcd = a.lc_dirs + (t << a.lc_log2n);
   }
   unsigned long long kept = 0;
-  // a half's fate waits on its length (distthresh), on the avoid mask, or on the waypoints both
-  // halves passed (Seedmanager::run keeps a first half with reject flag 2 when the second half
-  // completes the waypoints)
-  const bool decide = a.o.distthresh > 0.f || a.v.avoid != nullptr || a.v.nwaypoints > 0;
+  uint32_t* const list0 = (FEAT & kFeatKeep) && a.lists ? a.lists + t * 2 * a.list_cap : nullptr;
   for (uint64_t pid = a.pid_begin + t; pid < a.pid_end; pid += threads) {
     T.stamp = (uint32_t)(pid - a.pid_begin) + 1u;
     const int s = (int)(pid / (uint64_t)a.o.nparticles);
@@ -575,13 +610,24 @@ __global__ void __launch_bounds__(kTrackThreads, kTrackBlocksPerSm) track_kernel
     uint32_t flags = 0;  // waypoints passed by both halves (Streamliner::reset clears them per particle)
     int nvisit = 0;      // distinct voxels counted so far (the first half's before the second's)
     Counted cnt{0.f, 0u, s, 0};
-    if (decide) {  // whether a half counts is known only once both halves have ended: track, then count
+    if (FEAT & kFeatKeep) {
+      // a half's fate waits on its length (distthresh), on the avoid mask, or on the waypoints both
+      // halves passed (Seedmanager::run keeps a first half with reject flag 2 when the second half
+      // completes the waypoints), so it counts only once both halves have ended
       const Particle P0 = P;
-      const int rej1 = T.template half_line<FEAT>(P, pid, 0, fibst, x0, y0, z0, false, flags, nvisit, cnt);
+      int n0 = 0, n1 = 0;
+      uint32_t* const list1 = list0 ? list0 + a.list_cap : nullptr;
+      const int rej1 = T.template half_line<FEAT>(P, pid, 0, fibst, x0, y0, z0, false, flags, nvisit, cnt, list0, &n0);
       reverse(P);
       const Particle P1 = P;
-      const int rej2 = T.template half_line<FEAT>(P, pid, 1, fibst, x0, y0, z0, false, flags, nvisit, cnt);
+      const int rej2 = T.template half_line<FEAT>(P, pid, 1, fibst, x0, y0, z0, false, flags, nvisit, cnt, list1, &n1);
       const bool fwd = (rej1 == 0 || rej1 == 2) && !(rej2 > 0 && rej1 > 0), bwd = rej2 == 0;
+      if (fwd || bwd) ++kept;
+      if (list0) {
+        if (fwd) T.template count_list<FEAT>(list0, n0, nvisit, cnt);
+        if (bwd) T.template count_list<FEAT>(list1, n1, nvisit, cnt);
+        continue;
+      }
       uint32_t unused = 0;
       if (fwd) {
         Particle Q = P0;
@@ -591,7 +637,6 @@ __global__ void __launch_bounds__(kTrackThreads, kTrackBlocksPerSm) track_kernel
         Particle Q = P1;
         T.template half_line<FEAT>(Q, pid, 1, fibst, x0, y0, z0, true, unused, nvisit, cnt);
       }
-      if (fwd || bwd) ++kept;
     } else {  // every half is kept: count as it goes
       T.template half_line<FEAT>(P, pid, 0, fibst, x0, y0, z0, true, flags, nvisit, cnt);
       reverse(P);
@@ -604,18 +649,47 @@ __global__ void __launch_bounds__(kTrackThreads, kTrackBlocksPerSm) track_kernel
   if ((threadIdx.x & 31) == 0 && kept) atomicAdd(a.waytotal, kept);
 }
 
+// track_kernel<FEAT> for every feature set
+template <int... F>
+constexpr auto track_kernels(std::integer_sequence<int, F...>) {
+  return std::array<void (*)(TrackArgs), sizeof...(F)>{track_kernel<F>...};
+}
+const auto kTrackKernels = track_kernels(std::make_integer_sequence<int, kFeats>{});
+
 // The samples [K][nsamples][nvox] of th, ph and f repacked as one record per (voxel, sample)
 // (TrackArgs::packed): a 32 x 32 tile of (voxel, sample) per block, read along voxels and written
 // along samples through shared memory, so both sides are coalesced.  Each fibre's direction is
-// formed here once, with the sine and cosine every step would otherwise form again.
+// formed here once, with the sine and cosine every step would otherwise form again.  A step samples a
+// voxel within `reach` voxels of a position whose own voxel is inside the mask, so tiles with no masked
+// voxel that near are left out (a brain fills under half of its grid; those records are never used).
+struct PackReach {
+  int x, y, z;  // negative x: every tile
+};
 constexpr int kPackTile = 32;
 __global__ void __launch_bounds__(256) pack_samples_kernel(const float* __restrict__ th, const float* __restrict__ ph,
-                                                           const float* __restrict__ f, int K, int ns, size_t nvox,
-                                                           int pk4, float4* __restrict__ out) {
+                                                           const float* __restrict__ f, const float* __restrict__ mask,
+                                                           int nx, int ny, int nz, PackReach reach, int K, int ns,
+                                                           size_t nvox, int pk4, float4* __restrict__ out) {
   __shared__ float tile[3 * BPX_MAX_FIBRES][kPackTile][kPackTile + 1];
   const size_t v0 = (size_t)blockIdx.x * kPackTile;
   const int s0 = blockIdx.y * kPackTile;
   const int tx = threadIdx.x, ty = threadIdx.y;
+  if (reach.x >= 0) {
+    const size_t vx = v0 + tx;
+    bool near = false;
+    if (vx < nvox) {
+      const int x = (int)(vx % nx), y = (int)(vx / nx % ny), z = (int)(vx / ((size_t)nx * ny));
+      // warp ty takes every eighth (y, z) row of the neighbourhood
+      const int rows_y = 2 * reach.y + 1, rows = rows_y * (2 * reach.z + 1);
+      for (int r = ty; r < rows && !near; r += blockDim.y) {
+        const int yy = y - reach.y + r % rows_y, zz = z - reach.z + r / rows_y;
+        if (yy < 0 || yy >= ny || zz < 0 || zz >= nz) continue;
+        const float* m = mask + ((size_t)zz * ny + yy) * nx;
+        for (int xx = max(0, x - reach.x); xx <= min(nx - 1, x + reach.x); ++xx) near |= __ldg(m + xx) > 0.f;
+      }
+    }
+    if (!__syncthreads_or(near)) return;
+  }
   for (int c = 0; c < 3 * K; ++c) {
     const float* src = (c % 3 == 0) ? th : (c % 3 == 1) ? ph : f;
     const int k = c / 3;
@@ -761,37 +835,53 @@ bpx_status bpx_probtrack_dev(const bpx_track_options* opts, const bpx_track_volu
   // particles in flight: kTrackBlocksPerSm blocks per SM, fewer when the tables of very long paths
   // would pass 16 GB
   const size_t table_bytes = ((size_t)1 << log2n) * sizeof(uint2);
-  const size_t max_blocks = ((size_t)16 << 30) / ((table_bytes + lc_bytes) * kTrackThreads);
+  const bool keep = opts->distthresh > 0.f || vol->avoid != nullptr || vol->nwaypoints > 0;
+  // the lists of a particle's voxels, one per half with an entry per step at most; the counts that need
+  // more than the voxels are made by tracking the kept halves again
+  const bool list = keep && vol->m2_ncols == 0 && (vol->ntargets == 0 || !(opts->distthresh > 0.f));
+  a.list_cap = (size_t)(opts->nsteps / 2);
+  const size_t list_bytes = list ? 2 * a.list_cap * sizeof(uint32_t) : 0;
+  const size_t max_blocks = ((size_t)16 << 30) / ((table_bytes + lc_bytes + list_bytes) * kTrackThreads);
   const int feat = (opts->modeuler ? kFeatEuler : 0) | (opts->loopcheck ? kFeatLoop : 0) |
                    ((vol->ntargets > 0 || vol->m2_ncols > 0 || vol->m1_ncols > 0) ? kFeatCount : 0) |
-                   (vol->prefdir ? kFeatPref : 0);
+                   (vol->prefdir ? kFeatPref : 0) | (keep ? kFeatKeep : 0);
+  const uint64_t total = (uint64_t)nseeds * (uint64_t)opts->nparticles;
   int grid = sm_count() * kTrackBlocksPerSm;
   if ((size_t)grid > max_blocks) grid = max_blocks > 0 ? (int)max_blocks : 1;
+  // no more threads than particles: the tables, which are cleared for every call, shrink with the call
+  // (4 seeds x 5000 particles: 0.7 ms of clearing 5 GB against 0.1 ms)
+  const uint64_t want = (total + kTrackThreads - 1) / kTrackThreads;
+  if (want < (uint64_t)grid) grid = (int)want;
   const size_t threads = (size_t)grid * kTrackThreads;
   // workspace: the visit tables, the loopcheck tables (keys, then directions), the repacked samples
   const int pk4 = vol->nfib + 1;
   const size_t tab_total = (threads * table_bytes + 255) & ~(size_t)255;
   const size_t lc_keys = opts->loopcheck ? (threads * ((size_t)1 << lc_log2n) * sizeof(uint2) + 255) & ~(size_t)255 : 0;
   const size_t lc_dirs = opts->loopcheck ? threads * ((size_t)1 << lc_log2n) * sizeof(float4) : 0;
+  const size_t lists_total = (threads * list_bytes + 255) & ~(size_t)255;
   const size_t packed_bytes = a.nvox * (size_t)vol->nsamples * (size_t)pk4 * sizeof(float4);
   void* ws = nullptr;
-  st = api_workspace(kWsTrack, tab_total + lc_keys + lc_dirs + packed_bytes, &ws);
+  st = api_workspace(kWsTrack, tab_total + lc_keys + lc_dirs + lists_total + packed_bytes, &ws);
   if (st != BPX_OK) return st;
   a.tables = (uint2*)ws;
   a.lc_keys = opts->loopcheck ? (uint2*)((char*)ws + tab_total) : nullptr;
   a.lc_dirs = opts->loopcheck ? (float4*)((char*)ws + tab_total + lc_keys) : nullptr;
-  a.packed = (const float4*)((char*)ws + tab_total + lc_keys + lc_dirs);
+  a.lists = list ? (uint32_t*)((char*)ws + tab_total + lc_keys + lc_dirs) : nullptr;
+  a.packed = (const float4*)((char*)ws + tab_total + lc_keys + lc_dirs + lists_total);
   a.pk4 = pk4;
   cudaStream_t s = (cudaStream_t)stream;
   {
     const dim3 block(kPackTile, 8);
     const dim3 pgrid((unsigned)((a.nvox + kPackTile - 1) / kPackTile), (unsigned)((vol->nsamples + kPackTile - 1) / kPackTile));
-    pack_samples_kernel<<<pgrid, block, 0, s>>>(vol->th, vol->ph, vol->f, vol->nfib, vol->nsamples, a.nvox, pk4,
-                                                 (float4*)a.packed);
+    // |sampled voxel - position's voxel| < 1.5 (rounding either way), plus the test jump with --modeuler
+    const auto reach1 = [&](float step) { return opts->modeuler ? (int)std::floor(1.5 + (double)step * 1.001) : 1; };
+    PackReach reach{-1, 0, 0};
+    if (!opts->modeuler || fmaxf(a.sx, fmaxf(a.sy, a.sz)) <= 2.f) reach = PackReach{reach1(a.sx), reach1(a.sy), reach1(a.sz)};
+    pack_samples_kernel<<<pgrid, block, 0, s>>>(vol->th, vol->ph, vol->f, vol->mask, vol->nx, vol->ny, vol->nz, reach,
+                                                 vol->nfib, vol->nsamples, a.nvox, pk4, (float4*)a.packed);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return api_cuda_fail(e, "bpx_probtrack_dev: pack_samples_kernel");
   }
-  const uint64_t total = (uint64_t)nseeds * (uint64_t)opts->nparticles;
   const uint64_t chunk = 1ull << 30;  // stamps stay below 2^30 + 1 within a launch
   for (uint64_t b = 0; b < total; b += chunk) {
     // stamp 0 marks every entry empty before a launch reuses the tables
@@ -799,24 +889,7 @@ bpx_status bpx_probtrack_dev(const bpx_track_options* opts, const bpx_track_volu
     if (e0 != cudaSuccess) return api_cuda_fail(e0, "bpx_probtrack_dev: cudaMemsetAsync");
     a.pid_begin = b;
     a.pid_end = b + chunk < total ? b + chunk : total;
-    switch (feat) {
-      case 0: track_kernel<0><<<grid, kTrackThreads, 0, s>>>(a); break;
-      case 1: track_kernel<1><<<grid, kTrackThreads, 0, s>>>(a); break;
-      case 2: track_kernel<2><<<grid, kTrackThreads, 0, s>>>(a); break;
-      case 3: track_kernel<3><<<grid, kTrackThreads, 0, s>>>(a); break;
-      case 4: track_kernel<4><<<grid, kTrackThreads, 0, s>>>(a); break;
-      case 5: track_kernel<5><<<grid, kTrackThreads, 0, s>>>(a); break;
-      case 6: track_kernel<6><<<grid, kTrackThreads, 0, s>>>(a); break;
-      case 7: track_kernel<7><<<grid, kTrackThreads, 0, s>>>(a); break;
-      case 8: track_kernel<8><<<grid, kTrackThreads, 0, s>>>(a); break;
-      case 9: track_kernel<9><<<grid, kTrackThreads, 0, s>>>(a); break;
-      case 10: track_kernel<10><<<grid, kTrackThreads, 0, s>>>(a); break;
-      case 11: track_kernel<11><<<grid, kTrackThreads, 0, s>>>(a); break;
-      case 12: track_kernel<12><<<grid, kTrackThreads, 0, s>>>(a); break;
-      case 13: track_kernel<13><<<grid, kTrackThreads, 0, s>>>(a); break;
-      case 14: track_kernel<14><<<grid, kTrackThreads, 0, s>>>(a); break;
-      default: track_kernel<15><<<grid, kTrackThreads, 0, s>>>(a); break;
-    }
+    kTrackKernels[feat]<<<grid, kTrackThreads, 0, s>>>(a);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return api_cuda_fail(e, "bpx_probtrack_dev: track_kernel");
   }
