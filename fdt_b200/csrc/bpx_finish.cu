@@ -19,21 +19,27 @@
 namespace bpx {
 
 // principal eigenvector of a symmetric 3x3 (cyclic Jacobi, FP64), largest |component| positive;
-// returns the largest eigenvalue
+// returns the largest eigenvalue.  A rotation is a chain of long FP64 operations and few threads run it, so
+// it is bound by their latency: the tangent takes one square root and one division, the cosine one
+// reciprocal square root, and the sweeps end when the off-diagonal elements are below FP64 rounding of
+// the matrix (1e-16.5 of its norm) instead of at underflow.
 __device__ double principal_vector(double (&A)[3][3], double (&out)[3]) {
   double V[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
+  const double tol = 1e-33 * (A[0][0] * A[0][0] + A[1][1] * A[1][1] + A[2][2] * A[2][2] +
+                              2.0 * (A[0][1] * A[0][1] + A[0][2] * A[0][2] + A[1][2] * A[1][2]));
   for (int sweep = 0; sweep < 50; ++sweep) {
     const double off = A[0][1] * A[0][1] + A[0][2] * A[0][2] + A[1][2] * A[1][2];
-    if (off < 1e-300) break;
+    if (off <= tol) break;
 #pragma unroll
     for (int p = 0; p < 3; ++p)
 #pragma unroll
       for (int q = p + 1; q < 3; ++q) {
         const double apq = A[p][q];
-        if (fabs(apq) < 1e-300) continue;
-        const double theta = (A[q][q] - A[p][p]) / (2.0 * apq);
-        const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-        const double c = 1.0 / sqrt(t * t + 1.0), s = t * c;
+        if (apq * apq <= 0.1 * tol) continue;
+        const double b = A[q][q] - A[p][p], e = 2.0 * apq;
+        const double m = fabs(e) / (fabs(b) + sqrt(b * b + e * e));
+        const double t = (b == 0.0 || (b > 0.0) == (e > 0.0)) ? m : -m;
+        const double c = rsqrt(t * t + 1.0), s = t * c;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
           const double akp = A[k][p], akq = A[k][q];
