@@ -102,6 +102,7 @@ struct McmcArgs {
   const float* props_in;  // [6+3K][nvox] initial proposal widths, or NULL for initialise_props
   float* props_out;       // [6+3K][nvox] proposal widths after the last iteration, or NULL
   int freeze_props;       // 0: adapt (reference); 1: never adapt; 2: adapt during burn-in only
+  int spread;             // one voxel per warp whatever the layout (set by the launcher for small volumes)
   const uint64_t* voxel_keys;  // [nvox] RNG voxel keys (packed batches), or NULL: voxel_offset + v
   // a stretch of the chain: iterations [it_begin, it_end) (it_end 0: to the end), started from
   // state_in [6+3K][nvox] (record rows) and acc_in [6+3K][nvox] when given; the state, acceptance
