@@ -315,7 +315,7 @@ struct Tracker {
   // The voxel and posterior sample a step reads (the probabilistic rounding of Tractvolsx::sample):
   // depends only on the position and the step's uniforms, so its loads can be issued together
   // with the mask's.
-  __device__ void locate(float x, float y, float z, const float (&u)[8], size_t& vox, int& samp) const {
+  __device__ __forceinline__ void locate(float x, float y, float z, const float (&u)[8], size_t& vox, int& samp) const {
     const bpx_track_volume& v = a.v;
     const int cx = (int)ceilf(x), fx = (int)floorf(x);
     const int cy = (int)ceilf(y), fy = (int)floorf(y);
@@ -403,182 +403,208 @@ struct Tracker {
     f = a.o.usef ? ff : 1.0f;
   }
 
-  // Streamliner::streamline for one half; counts the path's first visits when `count` (with --pd
-  // the d-th distinct voxel of the particle adds d; nvisit carries d over the kept halves).  `flags`
-  // accumulates the waypoint masks passed (over both halves of a particle).  Returns the reject
-  // flag: 1 (entered the avoid mask, passed no waypoint, or shorter than distthresh), 2 (passed
-  // some waypoints but not all), 0.
-  // FEAT: the feature set compiled in (kFeatEuler, kFeatLoop, kFeatCount).  list: the voxels entered
-  // are written there instead (count false), their number to nlist.
-  template <int FEAT>
-  __device__ int half_line(Particle& P, uint64_t pid, int h, int fibst0, float x0, float y0, float z0,
-                           bool count, uint32_t& flags, int& nvisit, Counted& cnt, uint32_t* list = nullptr,
-                           int* nlist = nullptr) {
-    const bpx_track_options& o = a.o;
-    const bpx_track_volume& v = a.v;
-    bool init_sample = true, avoided = false;
-    int fibst = fibst0;
+  // ---- Streamliner::streamline for one half, a step at a time ----
+  // the state of a half besides the particle
+  struct Half {
+    int it;            // the next step (1-based)
+    int fibst;
+    uint32_t last, last_lr;
+    uint32_t lc_cell;  // --loopcheck: the coarse cell of the step before and the direction stored for
+    float3 lc_dir;     // it since; the table is read and written only when the cell changes (about every 20
+                       // steps of 0.5 mm in 2 mm voxels), which stores and finds the same directions as
+                       // a table access every step
+    float pathlength;
+    int nl;
+    bool init_sample, avoided;
+  };
+
+  __device__ __forceinline__ void begin_half(Half& H, Particle& P, int fibst0, float x0, float y0, float z0) {
     P.x = x0;
     P.y = y0;
     P.z = z0;
-    float pathlength = 0.f;
-    const int K = v.nfib;
+    H.it = 1;
+    H.fibst = fibst0;
     // a step of steplength mm mostly stays in the voxel of the step before, which is counted
     // already: the visit table is probed only when the voxel changes
-    uint32_t last = 0xffffffffu, last_lr = 0xffffffffu;
-    int nl = 0;
+    H.last = H.last_lr = H.lc_cell = 0xffffffffu;
+    H.lc_dir = make_float3(0.f, 0.f, 0.f);
+    H.pathlength = 0.f;
+    H.nl = 0;
+    H.init_sample = true;
+    H.avoided = false;
     ++lc_stamp;  // every tracked half starts with an empty loopcheck volume
-    // --loopcheck: the coarse cell of the step before and the direction stored for it since; the
-    // table is read and written only when the cell changes (about every 20 steps of 0.5 mm in 2 mm
-    // voxels), which stores and finds the same directions as a table access every step
-    uint32_t lc_cell = 0xffffffffu;
-    float3 lc_dir = make_float3(0.f, 0.f, 0.f);
-    for (int it = 1; it <= o.nsteps / 2; ++it) {
-      const int ix = rnd(P.x), iy = rnd(P.y), iz = rnd(P.z);
-      // this step's uniforms and sampled voxel, then the masks at the position and every fibre's
-      // sample in one round of loads (the reference reads them only inside the mask: same values)
-      // this step's uniforms: the first block always (rounding, sample); the second (randfib's
-      // draw, the --usef test, the first jump's sign) only while one of its draws can be used
-      float u[8], f;
-      uniform_block(o.seed, pid, h, (uint32_t)it, 0, u);
-      if (o.usef || !P.jumped || (init_sample && K > 1 && (o.randfib == 1 || o.randfib == 2))) {
-        uniform_block(o.seed, pid, h, (uint32_t)it, 1, u);
-      } else {
-        u[4] = u[5] = u[6] = u[7] = 0.f;  // f is 1 without --usef, so the step is taken
-      }
-      size_t svox;
-      int samp;
-      locate(P.x, P.y, P.z, u, svox, samp);
-      const bool in_grid = ix >= 0 && iy >= 0 && iz >= 0 && ix < v.nx && iy < v.ny && iz < v.nz;
-      const uint32_t vox = in_grid ? (uint32_t)(((size_t)iz * v.ny + iy) * v.nx + ix) : 0u;
-      const float m = __ldg(v.mask + vox);
-      const uint32_t way = v.waypoints ? __ldg(v.waypoints + vox) : 0u;
-      float3 pref = make_float3(0.f, 0.f, 0.f);  // --prefdir at the rounded position
-      if ((FEAT & kFeatPref) && v.prefdir)
-        pref = make_float3(__ldg(v.prefdir + vox), __ldg(v.prefdir + a.nvox + vox), __ldg(v.prefdir + 2 * a.nvox + vox));
-      // what the counting below reads, in the same round: the target bits of a new voxel, the
-      // matrix2 column of a new tract-space voxel (lr: its index, or ~0 off the tract-space grid)
-      uint32_t tgt = 0u, lr = 0xffffffffu;
-      int col = 0;
-      if ((FEAT & kFeatCount) && count) {
-        if (v.ntargets > 0 && vox != last) tgt = __ldg(v.targets + vox);
-        if (v.m2_ncols > 0) {
-          const int lx = lr_round(P.x, v.dx, v.lr_dx, a.lrx);
-          const int ly = lr_round(P.y, v.dy, v.lr_dy, a.lry);
-          const int lz = lr_round(P.z, v.dz, v.lr_dz, a.lrz);
-          if (lx >= 0 && ly >= 0 && lz >= 0 && lx < v.lr_nx && ly < v.lr_ny && lz < v.lr_nz) {
-            lr = ((uint32_t)lz * (uint32_t)v.lr_ny + (uint32_t)ly) * (uint32_t)v.lr_nx + (uint32_t)lx;
-            if (lr != last_lr) col = __ldg(v.m2_lookup + lr);
-          }
-        }
-      }
-      const bool avoid = v.avoid && __ldg(v.avoid + vox) != 0.f;
-      const bool stop = v.stop && __ldg(v.stop + vox) != 0.f;
-      Sample S;
-      load_record(svox, samp, S);
-      if (!(in_grid && m > 0.f)) break;  // the reference's remaining steps change nothing
-      if ((FEAT & kFeatLoop) && o.loopcheck) {
-        // stop where the path runs against the direction it last had in this coarse cell
-        const int lx = lc_round(P.x), ly = lc_round(P.y), lz = lc_round(P.z);
-        const uint32_t cell = ((uint32_t)lz * (uint32_t)a.lcny + (uint32_t)ly) * (uint32_t)a.lcnx + (uint32_t)lx;
-        float3 old = lc_dir;
-        if (cell != lc_cell) {
-          if (lc_cell != 0xffffffffu) loop_put(lc_cell, lc_dir);
-          old = loop_get(cell);
-          lc_cell = cell;
-        }
-        if (P.rx * old.x + P.ry * old.y + P.rz * old.z < 0.f) break;
-        lc_dir = make_float3(P.rx, P.ry, P.rz);
-      }
-      flags |= way;
-      if ((FEAT & kFeatKeep) && list && vox != last) {
-        last = vox;
-        list[nl++] = vox;  // at most one per step: the list holds nsteps / 2
-      }
-      if (count && vox != last) {
-        last = vox;
-        count_visit<FEAT>(vox, nvisit, cnt);
-        if ((FEAT & kFeatCount) && v.ntargets > 0) {
-          // a target is counted at its first entry on the counted path (a voxel change), if the path
-          // is by then at least distthresh long (Counter::update_seedcounts)
-          const uint32_t tb = tgt & ~cnt.tflags;
-          if (tb) {
-            if (cnt.length >= o.distthresh)
-              for (uint32_t b = tb; b; b &= b - 1) atomicAdd(v.seeds_to_targets + (size_t)(__ffs(b) - 1) * a.nseeds + cnt.seed, 1);
-            cnt.tflags |= tb;
-          }
-        }
-      }
-      if ((FEAT & kFeatCount) && count && lr != 0xffffffffu && lr != last_lr) {
-        // --omatrix2: the tract-space voxel of the position, counted once per particle when its
-        // column is not 0 (Counter::update_matrix2_row); it can change inside a diffusion voxel
-        last_lr = lr;
-        if (col > 0 && col < v.m2_ncols && first_visit(lr | kLrKey))
-          atomicAdd(v.matrix2 + (size_t)cnt.seed * v.m2_ncols + col, o.pathdist ? ++cnt.nvisit2 : 1);
-      }
-      if ((FEAT & kFeatCount) && count) cnt.length += o.steplength;
-      pathlength += o.steplength;
-      if (avoid) {
-        avoided = true;
-        break;
-      }
-      if (stop) break;
-      float3 rn;
-      bool moves;
-      choose(P, u, S, pref, init_sample, fibst, rn, moves, f);
-      if (f > u[5]) {
-        // (cos ph sin th, sin ph sin th, cos th): the record's vector, products commuted
-        const float rxn = rn.x, ryn = rn.y, rzn = rn.z;
-        if (P.jumped && !(fabsf(rxn * P.rx + ryn * P.ry + rzn * P.rz) > o.c_thr)) break;
-        if (moves) {
-          if (!(FEAT & kFeatEuler) || !o.modeuler) {
-            jump_dir(P, a, rxn, ryn, rzn, u[6]);
-          } else {
-            // Particle::testjump, a sample there, and the jump along the mean of both directions
-            // (mean_sph_pol, streamlines.cc:12-27, as the normalised sum or difference)
-            float w[8];
-            euler_uniforms(o.seed, pid, h, (uint32_t)it, !P.jumped, w);
-            int tsign;
-            if (P.jumped)
-              tsign = (rxn * P.rx + ryn * P.ry + rzn * P.rz) > 0.f ? 1 : -1;
-            else
-              tsign = w[4] > 0.5f ? 1 : -1;
-            const float ts = (float)tsign;
-            const float tx = P.x + ts * a.sx * rxn;
-            const float ty = P.y + ts * a.sy * ryn;
-            const float tz = P.z + ts * a.sz * rzn;
-            size_t tvox;
-            int tsamp;
-            locate(tx, ty, tz, w, tvox, tsamp);
-            Sample T2;
-            load_record(tvox, tsamp, T2);
-            float3 b;
-            bool moves2;
-            float f2;
-            choose(P, w, T2, pref, init_sample, fibst, b, moves2, f2);
-            const float bx = b.x, by = b.y, bz = b.z;
-            const float same = (rxn * bx + ryn * by + rzn * bz) > 0.f ? 1.0f : -1.0f;
-            const float mx = (rxn + same * bx) * 0.5f, my = (ryn + same * by) * 0.5f, mz = (rzn + same * bz) * 0.5f;
-            const float n = sqrtf(mx * mx + my * my + mz * mz);
-            if (n > 0.f)
-              jump_dir(P, a, mx / n, my / n, mz / n, u[6]);
-            else
-              jump_dir(P, a, rxn, ryn, rzn, u[6]);
-          }
+  }
+
+  // One step of half h; counts the path's first visits when `count` (with --pd the d-th distinct voxel
+  // of the particle adds d; nvisit carries d over the kept halves), or writes the voxels entered to
+  // `list`.  `flags` accumulates the waypoint masks passed (over both halves of a particle).  Returns
+  // false when the half ends.  FEAT: the feature set compiled in.
+  template <int FEAT>
+  __device__ __forceinline__ bool step(Half& H, Particle& P, uint64_t pid, int h, bool count, uint32_t& flags,
+                                       int& nvisit, Counted& cnt, uint32_t* list) {
+    const bpx_track_options& o = a.o;
+    const bpx_track_volume& v = a.v;
+    const int K = v.nfib;
+    const int it = H.it++;
+    const int ix = rnd(P.x), iy = rnd(P.y), iz = rnd(P.z);
+    // this step's uniforms and sampled voxel, then the masks at the position and every fibre's
+    // sample in one round of loads (the reference reads them only inside the mask: same values)
+    // this step's uniforms: the first block always (rounding, sample); the second (randfib's
+    // draw, the --usef test, the first jump's sign) only while one of its draws can be used
+    float u[8], f;
+    uniform_block(o.seed, pid, h, (uint32_t)it, 0, u);
+    if (o.usef || !P.jumped || (H.init_sample && K > 1 && (o.randfib == 1 || o.randfib == 2))) {
+      uniform_block(o.seed, pid, h, (uint32_t)it, 1, u);
+    } else {
+      u[4] = u[5] = u[6] = u[7] = 0.f;  // f is 1 without --usef, so the step is taken
+    }
+    size_t svox;
+    int samp;
+    locate(P.x, P.y, P.z, u, svox, samp);
+    const bool in_grid = ix >= 0 && iy >= 0 && iz >= 0 && ix < v.nx && iy < v.ny && iz < v.nz;
+    const uint32_t vox = in_grid ? (uint32_t)(((size_t)iz * v.ny + iy) * v.nx + ix) : 0u;
+    const float m = __ldg(v.mask + vox);
+    const uint32_t way = v.waypoints ? __ldg(v.waypoints + vox) : 0u;
+    float3 pref = make_float3(0.f, 0.f, 0.f);  // --prefdir at the rounded position
+    if ((FEAT & kFeatPref) && v.prefdir)
+      pref = make_float3(__ldg(v.prefdir + vox), __ldg(v.prefdir + a.nvox + vox), __ldg(v.prefdir + 2 * a.nvox + vox));
+    // what the counting below reads, in the same round: the target bits of a new voxel, the
+    // matrix2 column of a new tract-space voxel (lr: its index, or ~0 off the tract-space grid)
+    uint32_t tgt = 0u, lr = 0xffffffffu;
+    int col = 0;
+    if ((FEAT & kFeatCount) && count) {
+      if (v.ntargets > 0 && vox != H.last) tgt = __ldg(v.targets + vox);
+      if (v.m2_ncols > 0) {
+        const int lx = lr_round(P.x, v.dx, v.lr_dx, a.lrx);
+        const int ly = lr_round(P.y, v.dy, v.lr_dy, a.lry);
+        const int lz = lr_round(P.z, v.dz, v.lr_dz, a.lrz);
+        if (lx >= 0 && ly >= 0 && lz >= 0 && lx < v.lr_nx && ly < v.lr_ny && lz < v.lr_nz) {
+          lr = ((uint32_t)lz * (uint32_t)v.lr_ny + (uint32_t)ly) * (uint32_t)v.lr_nx + (uint32_t)lx;
+          if (lr != H.last_lr) col = __ldg(v.m2_lookup + lr);
         }
       }
     }
-    if ((FEAT & kFeatKeep) && list) *nlist = nl;
+    const bool avoid = v.avoid && __ldg(v.avoid + vox) != 0.f;
+    const bool stop = v.stop && __ldg(v.stop + vox) != 0.f;
+    Sample S;
+    load_record(svox, samp, S);
+    if (!(in_grid && m > 0.f)) return false;  // the reference's remaining steps change nothing
+    if ((FEAT & kFeatLoop) && o.loopcheck) {
+      // stop where the path runs against the direction it H.last had in this coarse cell
+      const int lx = lc_round(P.x), ly = lc_round(P.y), lz = lc_round(P.z);
+      const uint32_t cell = ((uint32_t)lz * (uint32_t)a.lcny + (uint32_t)ly) * (uint32_t)a.lcnx + (uint32_t)lx;
+      float3 old = H.lc_dir;
+      if (cell != H.lc_cell) {
+        if (H.lc_cell != 0xffffffffu) loop_put(H.lc_cell, H.lc_dir);
+        old = loop_get(cell);
+        H.lc_cell = cell;
+      }
+      if (P.rx * old.x + P.ry * old.y + P.rz * old.z < 0.f) return false;
+      H.lc_dir = make_float3(P.rx, P.ry, P.rz);
+    }
+    flags |= way;
+    if ((FEAT & kFeatKeep) && list && vox != H.last) {
+      H.last = vox;
+      list[H.nl++] = vox;  // at most one per step: the list holds nsteps / 2
+    }
+    if (count && vox != H.last) {
+      H.last = vox;
+      count_visit<FEAT>(vox, nvisit, cnt);
+      if ((FEAT & kFeatCount) && v.ntargets > 0) {
+        // a target is counted at its first entry on the counted path (a voxel change), if the path
+        // is by then at least distthresh long (Counter::update_seedcounts)
+        const uint32_t tb = tgt & ~cnt.tflags;
+        if (tb) {
+          if (cnt.length >= o.distthresh)
+            for (uint32_t b = tb; b; b &= b - 1) atomicAdd(v.seeds_to_targets + (size_t)(__ffs(b) - 1) * a.nseeds + cnt.seed, 1);
+          cnt.tflags |= tb;
+        }
+      }
+    }
+    if ((FEAT & kFeatCount) && count && lr != 0xffffffffu && lr != H.last_lr) {
+      // --omatrix2: the tract-space voxel of the position, counted once per particle when its
+      // column is not 0 (Counter::update_matrix2_row); it can change inside a diffusion voxel
+      H.last_lr = lr;
+      if (col > 0 && col < v.m2_ncols && first_visit(lr | kLrKey))
+        atomicAdd(v.matrix2 + (size_t)cnt.seed * v.m2_ncols + col, o.pathdist ? ++cnt.nvisit2 : 1);
+    }
+    if ((FEAT & kFeatCount) && count) cnt.length += o.steplength;
+    H.pathlength += o.steplength;
+    if (avoid) {
+      H.avoided = true;
+      return false;
+    }
+    if (stop) return false;
+    float3 rn;
+    bool moves;
+    choose(P, u, S, pref, H.init_sample, H.fibst, rn, moves, f);
+    if (f > u[5]) {
+      // (cos ph sin th, sin ph sin th, cos th): the record's vector, products commuted
+      const float rxn = rn.x, ryn = rn.y, rzn = rn.z;
+      if (P.jumped && !(fabsf(rxn * P.rx + ryn * P.ry + rzn * P.rz) > o.c_thr)) return false;
+      if (moves) {
+        if (!(FEAT & kFeatEuler) || !o.modeuler) {
+          jump_dir(P, a, rxn, ryn, rzn, u[6]);
+        } else {
+          // Particle::testjump, a sample there, and the jump along the mean of both directions
+          // (mean_sph_pol, streamlines.cc:12-27, as the normalised sum or difference)
+          float w[8];
+          euler_uniforms(o.seed, pid, h, (uint32_t)it, !P.jumped, w);
+          int tsign;
+          if (P.jumped)
+            tsign = (rxn * P.rx + ryn * P.ry + rzn * P.rz) > 0.f ? 1 : -1;
+          else
+            tsign = w[4] > 0.5f ? 1 : -1;
+          const float ts = (float)tsign;
+          const float tx = P.x + ts * a.sx * rxn;
+          const float ty = P.y + ts * a.sy * ryn;
+          const float tz = P.z + ts * a.sz * rzn;
+          size_t tvox;
+          int tsamp;
+          locate(tx, ty, tz, w, tvox, tsamp);
+          Sample T2;
+          load_record(tvox, tsamp, T2);
+          float3 b;
+          bool moves2;
+          float f2;
+          choose(P, w, T2, pref, H.init_sample, H.fibst, b, moves2, f2);
+          const float bx = b.x, by = b.y, bz = b.z;
+          const float same = (rxn * bx + ryn * by + rzn * bz) > 0.f ? 1.0f : -1.0f;
+          const float mx = (rxn + same * bx) * 0.5f, my = (ryn + same * by) * 0.5f, mz = (rzn + same * bz) * 0.5f;
+          const float n = sqrtf(mx * mx + my * my + mz * mz);
+          if (n > 0.f)
+            jump_dir(P, a, mx / n, my / n, mz / n, u[6]);
+          else
+            jump_dir(P, a, rxn, ryn, rzn, u[6]);
+        }
+      }
+    }
+    return H.it <= o.nsteps / 2;
+  }
+
+  // The reject flag of an ended half: 1 (entered the avoid mask, passed no waypoint, or shorter than
+  // distthresh), 2 (passed some waypoints but not all), 0.
+  __device__ __forceinline__ int reject(const Half& H, uint32_t flags) const {
+    const bpx_track_volume& v = a.v;
     int rej = 0;
     if (v.nwaypoints > 0) {
       const uint32_t all = v.nwaypoints >= 32 ? 0xffffffffu : ((1u << v.nwaypoints) - 1u);
       const int passed = __popc(flags & all);
       rej = passed == 0 ? 1 : (passed < v.nwaypoints ? 2 : 0);
     }
-    if (avoided || pathlength < o.distthresh) rej = 1;
+    if (H.avoided || H.pathlength < a.o.distthresh) rej = 1;
     return rej;
   }
 };
+
+// Every thread walks its particles (pid_begin + thread, then one grid further each time), both halves of
+// each.  The halves of a warp's lanes end at different steps, so the steps are the warp's one loop and
+// a lane whose half has ended begins its next one there, instead of waiting for the warp's longest
+// (512 seeds x 5000 particles: 21.2 -> 17.3 ms).  With kFeatKeep an ended half can lead to counting its
+// list, which is long for one lane alone: the warp then waits until kRefillKeep lanes have ended
+// (distthresh on that field, 128 seeds: 10.8 ms with 1, 9.1 ms with 8; without lists 8 cost 26 ms
+// against 17.5: the lanes that wait are then the loss).
+constexpr int kRefillKeep = 8;
 
 template <int FEAT>
 __global__ void __launch_bounds__(kTrackThreads, kTrackBlocksPerSm) track_kernel(TrackArgs a) {
@@ -591,58 +617,108 @@ __global__ void __launch_bounds__(kTrackThreads, kTrackBlocksPerSm) track_kernel
   }
   unsigned long long kept = 0;
   uint32_t* const list0 = (FEAT & kFeatKeep) && a.lists ? a.lists + t * 2 * a.list_cap : nullptr;
-  for (uint64_t pid = a.pid_begin + t; pid < a.pid_end; pid += threads) {
-    T.stamp = (uint32_t)(pid - a.pid_begin) + 1u;
-    const int s = (int)(pid / (uint64_t)a.o.nparticles);
-    if (a.o.per_seed) T.paths = a.paths + (size_t)s * a.nvox;
-    float u0[8];
-    track_uniforms(a.o.seed, pid, 0, 0u, u0);  // the particle's own draws: step 0
-    int fibst = a.o.fibst - 1;
-    if (a.o.randfib > 2) fibst = rnd(u0[0] * (float)(a.v.nfib - 1));
-    fibst = clampi(fibst, 0, a.v.nfib - 1);
-    float x0 = a.seeds[3 * s], y0 = a.seeds[3 * s + 1], z0 = a.seeds[3 * s + 2];
-    if (a.o.sampvox) {
-      x0 += u0[1] - 0.5f;
-      y0 += u0[2] - 0.5f;
-      z0 += u0[3] - 0.5f;
+  uint64_t pid = a.pid_begin + t;
+  Particle P{};
+  Tracker::Half H{};
+  uint32_t flags = 0;  // waypoints passed by both halves (Streamliner::reset clears them per particle)
+  int nvisit = 0;      // distinct voxels counted so far (the first half's before the second's)
+  Counted cnt{0.f, 0u, 0, 0};
+  // the pass a lane is in: 0 and 1 track the first and second half; with kFeatKeep and no lists 2 and 3
+  // track the kept ones again to count them; -1: its particle has not begun
+  int pass = -1, rej1 = 0, n0 = 0;
+  bool jumped1 = false, fwd = false, bwd = false;
+  bool active = false, more = pid < a.pid_end;
+  for (;;) {
+    const unsigned running = __ballot_sync(0xffffffffu, active), waiting = __ballot_sync(0xffffffffu, !active && more);
+    if (!(running | waiting)) break;
+    if (__popc(waiting) >= ((FEAT & kFeatKeep) ? kRefillKeep : 1) || !running) {
+      if (!active && more) {
+        // what the ended half leads to
+        if (FEAT & kFeatKeep) {
+          // a half's fate waits on its length (distthresh), on the avoid mask, or on the waypoints both
+          // halves passed (Seedmanager::run keeps a first half with reject flag 2 when the second half
+          // completes the waypoints), so it counts only once both halves have ended
+          if (pass == 0) {
+            rej1 = T.reject(H, flags);
+            n0 = H.nl;
+          } else if (pass == 1) {
+            const int rej2 = T.reject(H, flags);
+            fwd = (rej1 == 0 || rej1 == 2) && !(rej2 > 0 && rej1 > 0);
+            bwd = rej2 == 0;
+            if (fwd || bwd) ++kept;
+            if (list0) {
+              if (fwd) T.template count_list<FEAT>(list0, n0, nvisit, cnt);
+              if (bwd) T.template count_list<FEAT>(list0 + a.list_cap, H.nl, nvisit, cnt);
+              fwd = bwd = false;
+            }
+          }
+        } else if (pass == 1) {
+          ++kept;  // every half is kept: counted as it went
+        }
+        // the next pass
+        if (pass == 0) {
+          reverse(P);
+          jumped1 = P.jumped;
+          pass = 1;
+        } else if ((FEAT & kFeatKeep) && pass == 1 && fwd) {
+          pass = 2;
+        } else if ((FEAT & kFeatKeep) && (pass == 1 || pass == 2) && bwd) {
+          pass = 3;
+        } else {  // the next particle
+          if (pass >= 0) pid += threads;
+          more = pid < a.pid_end;
+          pass = 0;
+        }
+        if (more) {
+          if (pass == 0) {
+            const int s = pid < (1ull << 32) ? (int)((uint32_t)pid / (uint32_t)a.o.nparticles)
+                                             : (int)(pid / (uint64_t)a.o.nparticles);
+            T.stamp = (uint32_t)(pid - a.pid_begin) + 1u;
+            cnt = Counted{0.f, 0u, s, 0};
+            if (a.o.per_seed) T.paths = a.paths + (size_t)s * a.nvox;
+          }
+          int fibst = a.o.fibst - 1;
+          float x0 = a.seeds[3 * cnt.seed], y0 = a.seeds[3 * cnt.seed + 1], z0 = a.seeds[3 * cnt.seed + 2];
+          if (a.o.randfib > 2 || a.o.sampvox) {
+            float u0[8];
+            track_uniforms(a.o.seed, pid, 0, 0u, u0);  // the particle's own draws: step 0
+            if (a.o.randfib > 2) fibst = rnd(u0[0] * (float)(a.v.nfib - 1));
+            if (a.o.sampvox) {
+              x0 += u0[1] - 0.5f;
+              y0 += u0[2] - 0.5f;
+              z0 += u0[3] - 0.5f;
+            }
+          }
+          fibst = clampi(fibst, 0, a.v.nfib - 1);
+          if (pass == 0) {
+            P = Particle{};
+            flags = 0;
+            nvisit = 0;
+          } else if ((FEAT & kFeatKeep) && pass == 2) {
+            const float rxi = P.rxi, ryi = P.ryi, rzi = P.rzi;  // the second half's start needs them again
+            P = Particle{};
+            P.rxi = rxi;
+            P.ryi = ryi;
+            P.rzi = rzi;
+          } else if ((FEAT & kFeatKeep) && pass == 3) {  // as reverse() left it after the first half
+            P.jumped = jumped1;
+            P.rx = jumped1 ? -P.rxi : 0.f;
+            P.ry = jumped1 ? -P.ryi : 0.f;
+            P.rz = jumped1 ? -P.rzi : 0.f;
+          }
+          T.begin_half(H, P, fibst, x0, y0, z0);
+          active = true;
+        }
+      }
+      __syncwarp();
     }
-    Particle P{};
-    uint32_t flags = 0;  // waypoints passed by both halves (Streamliner::reset clears them per particle)
-    int nvisit = 0;      // distinct voxels counted so far (the first half's before the second's)
-    Counted cnt{0.f, 0u, s, 0};
-    if (FEAT & kFeatKeep) {
-      // a half's fate waits on its length (distthresh), on the avoid mask, or on the waypoints both
-      // halves passed (Seedmanager::run keeps a first half with reject flag 2 when the second half
-      // completes the waypoints), so it counts only once both halves have ended
-      const Particle P0 = P;
-      int n0 = 0, n1 = 0;
-      uint32_t* const list1 = list0 ? list0 + a.list_cap : nullptr;
-      const int rej1 = T.template half_line<FEAT>(P, pid, 0, fibst, x0, y0, z0, false, flags, nvisit, cnt, list0, &n0);
-      reverse(P);
-      const Particle P1 = P;
-      const int rej2 = T.template half_line<FEAT>(P, pid, 1, fibst, x0, y0, z0, false, flags, nvisit, cnt, list1, &n1);
-      const bool fwd = (rej1 == 0 || rej1 == 2) && !(rej2 > 0 && rej1 > 0), bwd = rej2 == 0;
-      if (fwd || bwd) ++kept;
-      if (list0) {
-        if (fwd) T.template count_list<FEAT>(list0, n0, nvisit, cnt);
-        if (bwd) T.template count_list<FEAT>(list1, n1, nvisit, cnt);
-        continue;
-      }
-      uint32_t unused = 0;
-      if (fwd) {
-        Particle Q = P0;
-        T.template half_line<FEAT>(Q, pid, 0, fibst, x0, y0, z0, true, unused, nvisit, cnt);
-      }
-      if (bwd) {
-        Particle Q = P1;
-        T.template half_line<FEAT>(Q, pid, 1, fibst, x0, y0, z0, true, unused, nvisit, cnt);
-      }
-    } else {  // every half is kept: count as it goes
-      T.template half_line<FEAT>(P, pid, 0, fibst, x0, y0, z0, true, flags, nvisit, cnt);
-      reverse(P);
-      T.template half_line<FEAT>(P, pid, 1, fibst, x0, y0, z0, true, flags, nvisit, cnt);
-      ++kept;
+    if (active) {
+      const int h = (FEAT & kFeatKeep) ? pass & 1 : pass;
+      const bool count = !(FEAT & kFeatKeep) || pass >= 2;
+      active = T.template step<FEAT>(H, P, pid, h, count, flags, nvisit, cnt,
+                                     ((FEAT & kFeatKeep) && list0) ? list0 + h * a.list_cap : nullptr);
     }
+    __syncwarp();
   }
   // waytotal: one atomic per warp
   for (int o = 16; o >= 1; o >>= 1) kept += __shfl_xor_sync(0xffffffffu, kept, o);
@@ -678,7 +754,8 @@ __global__ void __launch_bounds__(256) pack_samples_kernel(const float* __restri
     const size_t vx = v0 + tx;
     bool near = false;
     if (vx < nvox) {
-      const int x = (int)(vx % nx), y = (int)(vx / nx % ny), z = (int)(vx / ((size_t)nx * ny));
+      const uint32_t i = (uint32_t)vx, r0 = i / (uint32_t)nx;  // nvox < 2^32
+      const int x = (int)(i - r0 * (uint32_t)nx), z = (int)(r0 / (uint32_t)ny), y = (int)(r0 - (uint32_t)z * (uint32_t)ny);
       // warp ty takes every eighth (y, z) row of the neighbourhood
       const int rows_y = 2 * reach.y + 1, rows = rows_y * (2 * reach.z + 1);
       for (int r = ty; r < rows && !near; r += blockDim.y) {
