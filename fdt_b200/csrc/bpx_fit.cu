@@ -681,6 +681,10 @@ __device__ bool lm_run(const Meas& ms, Real (&p)[LmShape<KIND, K, F0>::P], int l
   return stopped;
 }
 
+}  // namespace bpx
+#include "bpx_fit_single.cuh"
+namespace bpx {
+
 // adjacent-swap sort of fibres by decreasing f (sort_PVM_*, CUDA/PVM_single.cu:86-104)
 template <int K, int O, int P>
 __device__ __forceinline__ void sort_fibres(Real (&p)[P]) {
@@ -1009,10 +1013,10 @@ __device__ __forceinline__ bool needs_refit(const Real (&p)[P], int of1) {
 }
 
 template <int K, bool F0>
-__device__ void stage_start(const FitArgs& a, int v, int lane, double* st) {
+__device__ void stage_start(const FitArgs& a, int v, int lane, SingleFit& c) {
   const VoxelMeas vm(a, v);
   const Meas& ms = vm.ms;
-  const Real R = a.R, invR = 1.0 / (2.0 * R + 1.0);
+  c.ms = ms;
   double* res = a.scratch + (size_t)v * 16;
   bool bad = false;
   for (int m = lane; m < ms.M; m += 32) bad |= !isfinite(ms.y[m]);
@@ -1027,14 +1031,14 @@ __device__ void stage_start(const FitArgs& a, int v, int lane, double* st) {
   if (a.model == 1 && !a.nonlin) {
     Real p[LmShape<kSingleC, K, F0>::P];
     start_single_c<K, F0>(dt, ms, lane, p);
-    if (!lm_run<kSingleC, K, F0>(ms, p, lane, 0, R, invR, st)) flag = kFitCapped;
+    if (!single_lm_run<kSingleC, K, F0>(c, p)) flag = kFitCapped;
     finalise<kSingleC, K, F0>(p);
     if (F0 && needs_refit(p, 2)) flag |= kFitRefit;
     store_res(res, p, lane);
   } else {
     Real p[LmShape<kSingle, K, F0>::P];
     start_single<K, F0>(dt, p);
-    if (!lm_run<kSingle, K, F0>(ms, p, lane, 0, R, invR, st)) flag = kFitCapped;
+    if (!single_lm_run<kSingle, K, F0>(c, p)) flag = kFitCapped;
     finalise<kSingle, K, F0>(p);
     if (a.model == 1 && F0 && needs_refit(p, 2)) flag |= kFitRefit;
     store_res(res, p, lane);
@@ -1175,8 +1179,26 @@ __device__ __forceinline__ void run_stage(const FitArgs& a, unsigned int* queue,
 }
 
 template <int K, bool F0>
-__global__ void __launch_bounds__(kFitThreads, kFitMinBlocks) fit_start_kernel(FitArgs a, unsigned int* queue) {
-  run_stage(a, queue, [](const FitArgs& x, int v, int lane, double* st) { stage_start<K, F0>(x, v, lane, st); });
+__global__ void __launch_bounds__(kFitThreads, kFitStartMinBlocks) fit_start_kernel(FitArgs a, unsigned int* queue) {
+  extern __shared__ __align__(16) unsigned char start_smem[];
+  BTable& bt = *reinterpret_cast<BTable*>(start_smem);
+  unsigned char* bidx = start_smem + sizeof(BTable);
+  build_btable(a, bt, bidx);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int warps = gridDim.x * (kFitThreads / 32);
+  SingleFit c;
+  c.bt = &bt;
+  c.bidx = bidx;
+  c.w = reinterpret_cast<WarpMem*>(start_smem + single_block_bytes(a.ndir) + w * single_warp_bytes(K, a.ndir));
+  c.lcache = reinterpret_cast<Real*>(c.w + 1);
+  c.lane = lane;
+  int v = blockIdx.x * (kFitThreads / 32) + w;
+  while (v < a.nvox) {
+    stage_start<K, F0>(a, v, lane, c);
+    unsigned int n = 0;
+    if (lane == 0) n = atomicAdd(queue, 1u);
+    v = warps + (int)__shfl_sync(0xffffffffu, n, 0);
+  }
 }
 template <int K, bool F0>
 __global__ void __launch_bounds__(kFitThreads, kFitMinBlocks) fit_multi_kernel(FitArgs a, unsigned int* queue) {
@@ -1219,14 +1241,16 @@ __global__ void __launch_bounds__(kFitThreads) prepare_kernel(int nvox, int ndir
 // launchers
 // ------------------------------------------------------------------------------------------
 // One stage over every voxel: as many blocks as fit the device at once, fewer for small volumes.
-static cudaError_t launch_stage(void (*kern)(FitArgs, unsigned int*), const FitArgs& a, unsigned int* queue,
+static cudaError_t launch_stage(void (*kern)(FitArgs, unsigned int*), const FitArgs& a, unsigned int* queue, size_t smem,
                                 cudaStream_t s) {
   int per_sm = 0;
-  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFitThreads, 0);
+  cudaError_t e = cudaSuccess;
+  if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFitThreads, smem);
   if (e != cudaSuccess) return e;
   const int cap = sm_count() * (per_sm > 0 ? per_sm : 1), warps = kFitThreads / 32;
   const int want = (int)(((long long)a.nvox + warps - 1) / warps);
-  kern<<<want < cap ? want : cap, kFitThreads, 0, s>>>(a, queue);
+  kern<<<want < cap ? want : cap, kFitThreads, smem, s>>>(a, queue);
   return cudaGetLastError();
 }
 
@@ -1236,10 +1260,11 @@ static cudaError_t launch_fit_kf(const FitArgs& a, cudaStream_t s) {
   static_assert(LmShape<kMulti, K, F0>::P <= 14, "scratch doubles 14 and 15 hold the voxel counters");
   unsigned int* queue = reinterpret_cast<unsigned int*>(a.scratch + 14);
   cudaError_t e = cudaMemsetAsync(queue, 0, 4 * sizeof(unsigned int), s);
-  if (e == cudaSuccess) e = launch_stage(fit_start_kernel<K, F0>, a, queue, s);
-  if (e == cudaSuccess && a.model >= 2) e = launch_stage(fit_multi_kernel<K, F0>, a, queue + 1, s);
-  if (e == cudaSuccess && F0) e = launch_stage(fit_refit_kernel<K>, a, queue + 2, s);
-  if (e == cudaSuccess) e = launch_stage(fit_finish_kernel<K, F0>, a, queue + 3, s);
+  const size_t smem = single_block_bytes(a.ndir) + (kFitThreads / 32) * single_warp_bytes(K, a.ndir);
+  if (e == cudaSuccess) e = launch_stage(fit_start_kernel<K, F0>, a, queue, smem, s);
+  if (e == cudaSuccess && a.model >= 2) e = launch_stage(fit_multi_kernel<K, F0>, a, queue + 1, 0, s);
+  if (e == cudaSuccess && F0) e = launch_stage(fit_refit_kernel<K>, a, queue + 2, 0, s);
+  if (e == cudaSuccess) e = launch_stage(fit_finish_kernel<K, F0>, a, queue + 3, 0, s);
   return e;
 }
 

@@ -24,6 +24,7 @@ constexpr int kFitThreads = 128;   // 4 warps, one voxel per warp at a time
 #define BPX_FIT_MIN_BLOCKS 4
 #endif
 constexpr int kFitMinBlocks = BPX_FIT_MIN_BLOCKS;  // register cap: 65536 / (128 * 4) = 128 per thread
+constexpr int kFitStartMinBlocks = 5;  // the first fit: 65536 / (128 * 5) = 102 per thread
 constexpr int kMcmcThreads = 128;  // 4 warps
 // Register cap of the MCMC kernel as resident blocks per SM: 4 (128 registers, 16 warps) for up to
 // 9 measurements per lane, 3 (168 registers, 12 warps) for more, where 128 registers spill in the
