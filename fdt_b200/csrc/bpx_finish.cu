@@ -185,18 +185,20 @@ __global__ void __launch_bounds__(kVox * kGroups, 3) finish_kernel(FinishArgs a)
   sum_groups<Q>(val, fin);
   if (!in) return;
   const double inv = 1.0 / ns;
-  if (g < K) {  // warp g: fibre g's mean and dyad, to its sorted slot
-    int o = 0;
+  if (g < K) {  // warp g: the mean and dyad of output position g
+    // the fibre that comes there: sums that are NaN compare with none, so positions can then hold two
+    // fibres (the later one counts) or none (fibre 0)
+    int src = 0;
 #pragma unroll
     for (int k = 0; k < K; ++k)
-      if (k == g) o = slot[k];
-    if (out.mean_f) out.mean_f[(size_t)o * nvox + v] = (float)(sumf[g][x] * inv);
+      if (slot[k] == g) src = k;
+    if (out.mean_f) out.mean_f[(size_t)g * nvox + v] = (float)(sumf[src][x] * inv);
     if (out.dyads) {
       double A[3][3], pv[3];
-      full_tensor(fin + 6 + 6 * g, x, 1.0, A);
+      full_tensor(fin + 6 + 6 * src, x, 1.0, A);
       principal_vector(A, pv);
 #pragma unroll
-      for (int r = 0; r < 3; ++r) out.dyads[((size_t)o * 3 + r) * nvox + v] = (float)pv[r];
+      for (int r = 0; r < 3; ++r) out.dyads[((size_t)g * 3 + r) * nvox + v] = (float)pv[r];
     }
   } else if (g == kGroups - 1) {
     float* mean[6] = {out.mean_d, out.mean_f0, out.mean_tau, out.mean_dstd, out.mean_R, out.mean_S0};
