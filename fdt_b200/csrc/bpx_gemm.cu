@@ -7,19 +7,22 @@
 // Operands are read by TMA straight from row-major global tensors in either orientation:
 //   * K-major  (the contraction index is the contiguous one): A = X[M][K], B = W[N][K];
 //   * MN-major (M resp. N is the contiguous one): A stored [K][M], B stored [K][N].
-// Both land in shared memory in the non-swizzled canonical layout of 8x(16 B) core matrices.  A
-// rank-3 tensor map over the row-major tensor, {8 contiguous elements, row, group of 8 columns}
-// with strides {row pitch, 16 B}, makes one TMA copy write a whole tile in that layout:
-//   K-major tile  [K/8 groups][rows][8]  -> LBO (K direction) = rows*16 B, SBO (rows) = 128 B
-//   MN-major tile [MN/8 groups][K][8]    -> LBO (K direction) = 128 B,    SBO (MN)   = K*16 B
+// A rank-2 tensor map copies boxes whose rows are 64 elements, one 128-byte swizzle span, so the copy
+// engine moves whole lines.  As 16-byte rows of an unswizzled core-matrix layout, which it also takes, the
+// copies were most of a tile's time: 36.0 against 23.2 us for 32768 rows, 256 columns, K = 256 with bias
+// and GELU (warps issuing 35% and 48% of the active cycles), and 333 against 215 us for the whole
+// inference of 65536 rows of 288 inputs.  A chunk of 64 along K is
+//   K-major tile   [rows][64]: 8-row atoms of 1024 B (SBO); the next 16 of K are 32 B further in the span
+//   MN-major tile  [MN/64][64 of K][64]: atoms of 8 along K (SBO 1024 B), the next 64 of MN 8192 B on (LBO);
+//                  the next 16 of K are two atoms (2048 B) further
 // One thread issues TMA and MMA (M = 128, N = tile width <= 256, K = 16 per instruction) through
 // an mbarrier ring of two to four stages; eight warps then read the accumulator (tcgen05.ld: warp w
 // the 32 TMEM lanes w%4, every second block of 32 columns) and run the epilogue.  Every mbarrier
 // wait is bounded (about a second), after which the kernel records an error code, waits (bounded) for
 // its own MMAs and releases its tensor memory.
 //
-// The network's contractions are 2 to 5 chunks deep, so a CTA's time is its epilogue (256 erff per row
-// of a 256-wide tile): bound by FP32 issue with too few warps, not by the tensor pipe.  Hence eight
+// The network's contractions are 2 to 5 chunks deep, so most of a CTA's time is its epilogue (256 erff per
+// row of a 256-wide tile): bound by FP32 issue and by the loads that precede it, not by the tensor pipe.  Hence eight
 // epilogue warps and two CTAs per SM, a tile width chosen so that the CTAs fill the device
 // (choose_ntile), and for the weight gradients, whose output is a few tiles but whose contraction is
 // the whole batch, a split of the contraction over CTAs (GemmArgs::split; the partial sums are added
@@ -40,6 +43,7 @@ namespace gemm {
 
 constexpr int kTileM = 128;
 constexpr int kChunkK = 64;
+constexpr int kSpan = 64;  // elements of a 128-byte swizzle span
 constexpr int kThreads = 256;
 constexpr int kMaxStages = 4;
 constexpr long long kWaitCycles = 2000000000ll;  // ~1 s at 2 GHz
@@ -70,19 +74,18 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   }
 }
 
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2,
-                                            uint32_t bar) {
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
       :
-      : "r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+      : "r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(bar)
       : "memory");
 }
 
-// shared-memory matrix descriptor: no swizzle, Blackwell descriptor version 1
+// shared-memory matrix descriptor: 128-byte swizzle, Blackwell descriptor version 1
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
   return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-         ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
+         ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46) | (2ull << 61);
 }
 
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
@@ -138,6 +141,11 @@ struct Batch {
 __host__ __device__ inline int tiles_m(const GemmArgs& g) { return (g.M + kTileM - 1) / kTileM; }
 __host__ __device__ inline int tiles_n(const GemmArgs& g) { return (g.N + g.ntile - 1) / g.ntile; }
 
+// a stage's bytes of B: an MN-major tile takes whole spans
+__host__ __device__ inline uint32_t b_stage_bytes(const GemmArgs& g) {
+  return (uint32_t)(g.b_mn && g.ntile < kSpan ? kSpan : g.ntile) * kChunkK * 2;
+}
+
 __global__ void __launch_bounds__(kThreads, 2) gemm_kernel(const __grid_constant__ Batch batch) {
   extern __shared__ __align__(1024) unsigned char dsmem[];
   int prob = 0;
@@ -150,7 +158,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_kernel(const __grid_constant
   const int bx = tile % tm, by = tile / tm % tn, bz = tile / (tm * tn);
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(dsmem) + 1023) & ~uintptr_t(1023));
   const int nt = g.ntile;
-  const uint32_t a_bytes = kTileM * kChunkK * 2, b_bytes = (uint32_t)nt * kChunkK * 2;
+  const uint32_t a_bytes = kTileM * kChunkK * 2, b_bytes = b_stage_bytes(g);
   const uint32_t stage_bytes = a_bytes + b_bytes;
   Smem* sm = reinterpret_cast<Smem*>(base + stages * stage_bytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -184,13 +192,15 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_kernel(const __grid_constant
       const uint32_t bar = smem_u32(&sm->full[s]);
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" : : "r"(bar), "r"(stage_bytes) : "memory");
       if (g.a_mn)
-        tma_load_3d(sa, &map_a, 0, kc * kChunkK, m0 / 8, bar);
+        for (int j = 0; j < kTileM / kSpan; ++j)
+          tma_load_2d(sa + j * kSpan * kChunkK * 2, &map_a, m0 + j * kSpan, kc * kChunkK, bar);
       else
-        tma_load_3d(sa, &map_a, 0, m0, kc * (kChunkK / 8), bar);
+        tma_load_2d(sa, &map_a, kc * kChunkK, m0, bar);
       if (g.b_mn)
-        tma_load_3d(sb, &map_b, 0, kc * kChunkK, n0 / 8, bar);
+        for (uint32_t j = 0; j * kSpan * kChunkK * 2 < b_bytes; ++j)
+          tma_load_2d(sb + j * kSpan * kChunkK * 2, &map_b, n0 + j * kSpan, kc * kChunkK, bar);
       else
-        tma_load_3d(sb, &map_b, 0, n0, kc * (kChunkK / 8), bar);
+        tma_load_2d(sb, &map_b, kc * kChunkK, n0, bar);
     };
     bool ok = true;
     for (int i = 0; i < stages && kc0 + i < kc1; ++i) load(kc0 + i, i);
@@ -205,10 +215,8 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_kernel(const __grid_constant
       const uint32_t sa = smem_u32(base + s * stage_bytes), sb = sa + a_bytes;
 #pragma unroll
       for (int ks = 0; ks < kChunkK / 16; ++ks) {
-        const uint64_t da = g.a_mn ? smem_desc(sa + ks * 256, 128, kChunkK * 16)
-                                   : smem_desc(sa + ks * 2 * kTileM * 16, kTileM * 16, 128);
-        const uint64_t db = g.b_mn ? smem_desc(sb + ks * 256, 128, kChunkK * 16)
-                                   : smem_desc(sb + ks * 2 * nt * 16, nt * 16, 128);
+        const uint64_t da = g.a_mn ? smem_desc(sa + ks * 2048, kSpan * kChunkK * 2, 1024) : smem_desc(sa + ks * 32, 0, 1024);
+        const uint64_t db = g.b_mn ? smem_desc(sb + ks * 2048, kSpan * kChunkK * 2, 1024) : smem_desc(sb + ks * 32, 0, 1024);
         mma_bf16(tmem, da, db, idesc, (kc != kc0) || ks != 0);
       }
       mma_commit(smem_u32(&sm->empty[s]));
@@ -396,23 +404,24 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// Tensor map over a row-major bf16 tensor [rows][cols] (leading dimension ld elements) viewed as
-// {8 contiguous elements, row, column group of 8}; box {8, box_rows, box_groups}.
-static bool make_map(CUtensorMap* m, const uint16_t* ptr, int rows, int cols, int ld, int box_rows, int box_groups) {
+// Tensor map over a row-major bf16 tensor [rows][cols] (leading dimension ld elements); box of one span
+// by box_rows, 128-byte swizzle.
+static bool make_map(CUtensorMap* m, const uint16_t* ptr, int rows, int cols, int ld, int box_rows) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
-  const cuuint64_t dims[3] = {8, (cuuint64_t)rows, (cuuint64_t)(cols / 8)};
-  const cuuint64_t strides[2] = {(cuuint64_t)ld * 2, 16};
-  const cuuint32_t box[3] = {8, (cuuint32_t)box_rows, (cuuint32_t)box_groups};
-  const cuuint32_t estr[3] = {1, 1, 1};
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+  const cuuint32_t box[2] = {kSpan, (cuuint32_t)box_rows};
+  const cuuint32_t estr[2] = {1, 1};
   std::memset(m, 0, sizeof(*m));
-  return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<uint16_t*>(ptr), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t*>(ptr), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// (narrower MN-major tiles of B still take a whole span)
 size_t smem_bytes(int ntile, int stages) {
-  return stages * (size_t)(kTileM * kChunkK * 2 + ntile * kChunkK * 2) + 1024 + sizeof(Smem) + 64;
+  return stages * (size_t)(kTileM * kChunkK * 2 + (ntile < kSpan ? kSpan : ntile) * kChunkK * 2) + 1024 + sizeof(Smem) + 64;
 }
 
 // Stages of the ring: as many as keep two CTAs on an SM (about 100 KB each) and the contraction can
@@ -475,10 +484,10 @@ cudaError_t launch(const GemmOperands* op, const GemmArgs* g, int problems, cuda
   for (int i = 0; i < problems; ++i) {
     *why = check(op[i], g[i]);
     if (*why) return cudaErrorInvalidValue;
-    const bool ok_a = g[i].a_mn ? make_map(&b.a[i], op[i].a, g[i].K, g[i].M, op[i].lda, kChunkK, kTileM / 8)
-                                : make_map(&b.a[i], op[i].a, g[i].M, g[i].K, op[i].lda, kTileM, kChunkK / 8);
-    const bool ok_b = g[i].b_mn ? make_map(&b.b[i], op[i].b, g[i].K, g[i].N, op[i].ldb, kChunkK, g[i].ntile / 8)
-                                : make_map(&b.b[i], op[i].b, g[i].N, g[i].K, op[i].ldb, g[i].ntile, kChunkK / 8);
+    const bool ok_a = g[i].a_mn ? make_map(&b.a[i], op[i].a, g[i].K, g[i].M, op[i].lda, kChunkK)
+                                : make_map(&b.a[i], op[i].a, g[i].M, g[i].K, op[i].lda, kTileM);
+    const bool ok_b = g[i].b_mn ? make_map(&b.b[i], op[i].b, g[i].K, g[i].N, op[i].ldb, kChunkK)
+                                : make_map(&b.b[i], op[i].b, g[i].N, g[i].K, op[i].ldb, g[i].ntile);
     if (!ok_a || !ok_b) {
       *why = "cuTensorMapEncodeTiled failed (driver entry point missing or unsupported tensor shape)";
       return cudaErrorInvalidValue;

@@ -144,6 +144,33 @@ def test_finish_with_nan_fractions(torch, nan):
         assert np.allclose(out["mean_f"][pos], s[src, np.arange(nvox)] / ns, rtol=1e-6, atol=0, equal_nan=True)
 
 
+@pytest.mark.parametrize("a_mn", [0, 1])
+@pytest.mark.parametrize("b_mn", [0, 1])
+@pytest.mark.parametrize("M,N,K", [(8, 8, 8), (40, 24, 72), (64, 64, 64), (72, 40, 56), (136, 264, 136), (320, 72, 328)])
+def test_gemm_at_the_edges_of_its_spans(torch, M, N, K, a_mn, b_mn):
+    """Operand tiles are copied in spans of 64 elements: spans partly and wholly outside the matrix, tiles
+    narrower than a span, contractions that end inside one.  FP32 sums of exact BF16 products differ from
+    64-bit ones by less than 1e-5 of the sum of magnitudes; the columns next to the matrix stay unread."""
+    from fdt_b200 import lib
+
+    g = torch.Generator(device="cpu").manual_seed(M + 3 * N + 7 * K)
+    A = torch.randn((M, K), generator=g).to(torch.bfloat16)
+    B = torch.randn((N, K), generator=g).to(torch.bfloat16)
+
+    def padded(x):  # rows 8 elements longer than the matrix, NaN past its end
+        out = torch.full((x.shape[0], x.shape[1] + 8), float("nan"), dtype=torch.bfloat16, device="cuda")
+        out[:, : x.shape[1]] = x.cuda()
+        return out
+
+    a, b = padded(A.t() if a_mn else A), padded(B.t() if b_mn else B)
+    c = lib.gemm_bf16(a, b, M, N, K, a_mn=bool(a_mn), b_mn=bool(b_mn))
+    torch.cuda.synchronize()
+    assert lib.poll_error() == 0
+    ref = A.double() @ B.double().t()
+    bound = 1e-5 * (A.double().abs() @ B.double().abs().t()) + 1e-6
+    assert bool(((c.cpu().double() - ref).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("batch", [1, 63, 65, 960, 961, 2049])
 def test_gradients_at_the_edges_of_the_batch_split(torch, batch):
     """From 16 chunks of 64 rows (961 rows) the weight gradients' contractions run in two parts.  The bounds
