@@ -106,9 +106,6 @@ struct Bucket {
   float* netout = nullptr;
   float* props = nullptr;
   uint16_t* wbf = nullptr;
-  uint16_t* act0 = nullptr;
-  uint16_t* act1 = nullptr;
-  int chunk = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;
 };
@@ -407,9 +404,9 @@ bpx_status bpx_batch_create(const bpx_options* opts, const bpx_item* items, int3
   std::vector<size_t> base(b->buckets.size());
   auto learned_bytes = [&](const Bucket& bk) -> size_t {
     if (!bk.mlp) return 0;
-    const size_t n = bk.n, nin = bpx_mlp_nin(bk.M), chunk = std::min<size_t>(n, 32768);
+    const size_t n = bk.n, nin = bpx_mlp_nin(bk.M);
     return a256(n * nin * 2) + a256(n * 4) + a256(n * BPX_MLP_NOUT * 4) + a256((6 + 3 * bk.K) * n * 4) +
-           a256(mlp_weight_elems(bk.M) * 2) + 2 * a256(chunk * BPX_MLP_WIDTH * 2);
+           a256(mlp_weight_elems(bk.M) * 2);
   };
   auto bucket_bytes = [&](const Bucket& bk) {
     const size_t n = bk.n, K = bk.K, P = 2 + 3 * K + (bk.model >= 2 ? 1 : 0) + (opts->f0 ? 1 : 0);
@@ -456,14 +453,11 @@ bpx_status bpx_batch_create(const bpx_options* opts, const bpx_item* items, int3
     bk.packed.dyads = (float*)take(3 * K * n * 4);
     if (!bk.mlp) bk.fit_scratch = take(n * kFitScratchBytes);
     if (bk.mlp) {
-      bk.chunk = (int)std::min<size_t>(n, 32768);
       bk.x = (uint16_t*)take(n * bpx_mlp_nin(bk.M) * 2);
       bk.s0hat = (float*)take(n * 4);
       bk.netout = (float*)take(n * BPX_MLP_NOUT * 4);
       bk.props = (float*)take((6 + 3 * K) * n * 4);
       bk.wbf = (uint16_t*)take(mlp_weight_elems(bk.M) * 2);
-      bk.act0 = (uint16_t*)take((size_t)bk.chunk * BPX_MLP_WIDTH * 2);
-      bk.act1 = (uint16_t*)take((size_t)bk.chunk * BPX_MLP_WIDTH * 2);
     }
     // voxel maps
     std::vector<uint64_t> keys(n);
@@ -524,7 +518,7 @@ bpx_status bpx_batch_create(const bpx_options* opts, const bpx_item* items, int3
       pv.bvals = bk.bvals;
       bpx_status ls = bpx_mlp_features_dev(&pv, 0, bk.x, bk.s0hat, bk.stream);
       if (ls == BPX_OK)
-        ls = mlp_forward_buffers(bk.M, bk.mlp, bk.n, bk.x, bk.netout, bk.wbf, bk.act0, bk.act1, bk.chunk, bk.stream);
+        ls = mlp_forward_buffers(bk.M, bk.mlp, bk.n, bk.x, bk.netout, bk.wbf, bk.stream);
       if (ls == BPX_OK)
         ls = bpx_mlp_decode_dev(&oi, bk.n, bk.netout, bk.s0hat, bk.params, bk.tau, bk.props, bk.status, bk.stream);
       if (ls != BPX_OK) {

@@ -60,18 +60,22 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok;
+}
+
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+  if (mbar_try(bar, parity)) return true;
   const long long t0 = clock64();
-  while (true) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
+  while (!mbar_try(bar, parity))
     if (clock64() - t0 > kWaitCycles) return false;
-  }
+  return true;
 }
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
@@ -121,6 +125,23 @@ __device__ __forceinline__ float gelu_grad(float z) {
 
 __device__ __forceinline__ uint16_t to_bf16(float x) {
   return __bfloat16_as_ushort(__float2bfloat16_rn(x));
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
+  return (uint32_t)__bfloat16_as_ushort(p.x) | ((uint32_t)__bfloat16_as_ushort(p.y) << 16);
+}
+
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
 }
 
 struct Smem {
@@ -385,6 +406,246 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_kernel(const __grid_constant
 }
 
 // ---------------------------------------------------------------------------------------------
+// A chain of layers (network inference): every layer of 128 rows in one CTA
+// ---------------------------------------------------------------------------------------------
+// Bound by the FP32 issue of the epilogues (a GELU per element and hidden layer).  The rows' activations
+// stay in shared memory, as the spans the next layer's products read; the weights (0.5 MB for all
+// layers, L2-resident) pass through a ring of pieces of 64 along K by up to 128 output columns.  One
+// CTA has an SM to itself, so that the ring holds a whole layer, which lands during the epilogue of
+// the layer before, and the sums have two places in tensor memory: a layer's products of a span
+// begin when the epilogue has written that span, and only the last span's are waited for.
+// Inference of 65536 rows of 288 inputs: 215 us as five launches per 32768 rows (which wrote and read
+// their activations, 2 x 16 MB, and waited for copies in every tile), 162 us so; 5000 rows 74 and 59 us,
+// 300 rows 60 and 54 us.  Two CTAs of 128 rows to an SM with a ring of three pieces and one place for the
+// sums measured 160, 74 and 70 us.  Warps issue 59% of the active cycles; what is left is layer 0's copies
+// at a tile's start and the rounding of the tiles to whole rounds of the SMs.
+// The products of a tile are those of gemm_kernel in the same order, so the results are too.
+constexpr int kPieceN = 128;
+constexpr int kRing = 10;
+constexpr int kEpiWarps = 16;
+constexpr int kChainThreads = 32 * kEpiWarps + 64;  // a warp that issues the copies, one for the products
+constexpr int kBlockN = 16;                         // columns of a span that a warp takes
+constexpr int kSpanBytes = kTileM * kSpan * 2;
+constexpr int kActSpans = kChainWidth / kSpan;
+static_assert(kSpanBytes == kPieceN * kChunkK * 2, "a span of activations is as large as a piece of weights");
+static_assert(kEpiWarps == kTileM / 32 * (kSpan / kBlockN), "the epilogue warps cover a span");
+
+struct Chain {
+  CUtensorMap x, w[kChainLayers];
+  const float* bias[kChainLayers];
+  float* out;
+  int* error;
+  int rows, nin;
+};
+
+__device__ __forceinline__ float4 bias4(const float* b, bool vec) {
+  if (vec) return __ldg(reinterpret_cast<const float4*>(b));
+  return make_float4(__ldg(b), __ldg(b + 1), __ldg(b + 2), __ldg(b + 3));
+}
+
+struct ChainBars {
+  uint64_t full[kRing], empty[kRing], written[kActSpans], done, drained;
+  uint32_t tmem_base;
+  int failed;
+};
+
+constexpr size_t kChainSmem = (size_t)(kActSpans + kRing) * kSpanBytes + sizeof(ChainBars);
+static_assert(kChainSmem <= 227 * 1024, "shared memory of a CTA");
+
+// a bounded wait that also ends when another one has given up
+__device__ __forceinline__ bool chain_wait(ChainBars* sm, const uint64_t* bar, uint32_t parity) {
+  const uint32_t addr = smem_u32(bar);
+  if (mbar_try(addr, parity)) return true;
+  const long long t0 = clock64();
+  while (!mbar_try(addr, parity)) {
+    if (*(volatile int*)&sm->failed) return false;
+    if (clock64() - t0 > kWaitCycles) {
+      *(volatile int*)&sm->failed = 1;
+      return false;
+    }
+  }
+  return true;
+}
+
+// Pieces come in order of use: layer, chunk of K, half of the columns (the last layer, of kChainOut
+// columns, has one).  Piece p takes ring slot p % kRing.  One thread copies, another multiplies: a single
+// one, which also divided for slots and rounds, took 1300 cycles a piece, 3000 beside busy epilogue
+// warps, and was the kernel's bound (205 us for the 65536 rows).
+__device__ __forceinline__ int chain_chunks(int layer, int nk0) { return layer == 0 ? nk0 : kActSpans; }
+__device__ __forceinline__ int chain_halves(int layer) { return layer == kChainLayers - 1 ? 1 : kChainWidth / kPieceN; }
+
+__device__ __forceinline__ bool chain_copy(const Chain& c, ChainBars* sm, uint32_t act, uint32_t ring, int m0, int nk0,
+                                           int* copied) {
+  int p = 0, slot = 0;
+  uint32_t ph = 1;  // of the slot's previous piece; the first round finds its slots empty
+  for (int layer = 0; layer < kChainLayers; ++layer) {
+    const int halves = chain_halves(layer), nk = chain_chunks(layer, nk0);
+    const uint32_t w_bytes = halves == 1 ? kChainOut * kChunkK * 2 : kSpanBytes;
+    for (int kc = 0; kc < nk; ++kc)
+      for (int half = 0; half < halves; ++half) {
+        *copied = p;
+        if (p >= kRing && !chain_wait(sm, &sm->empty[slot], ph)) return false;
+        const bool with_x = layer == 0 && half == 0;
+        if (with_x && kc >= kActSpans) {  // the chunk that was in this span
+          const int q = p - 2 * kActSpans + 1;
+          if (!chain_wait(sm, &sm->empty[q % kRing], (q / kRing) & 1)) return false;
+        }
+        const uint32_t bar = smem_u32(&sm->full[slot]), bytes = w_bytes + (with_x ? kSpanBytes : 0);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" : : "r"(bar), "r"(bytes) : "memory");
+        if (with_x) tma_load_2d(act + (kc % kActSpans) * kSpanBytes, &c.x, kc * kChunkK, m0, bar);
+        tma_load_2d(ring + slot * kSpanBytes, &c.w[layer], kc * kChunkK, half * kPieceN, bar);
+        ++p;
+        if (++slot == kRing) {
+          slot = 0;
+          ph ^= 1;
+        }
+      }
+  }
+  *copied = p;
+  return true;
+}
+
+__device__ __forceinline__ bool chain_multiply(ChainBars* sm, uint32_t act, uint32_t ring, uint32_t tmem, int nk0) {
+  int slot = 0;
+  uint32_t ph = 0;
+  const uint64_t act_desc = smem_desc(act, 0, 1024), ring_desc = smem_desc(ring, 0, 1024);
+  for (int layer = 0; layer < kChainLayers; ++layer) {
+    const int halves = chain_halves(layer), nk = chain_chunks(layer, nk0), n = halves == 1 ? kChainOut : kPieceN;
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
+    const uint32_t sums = tmem + (layer & 1) * kChainWidth;
+    for (int kc = 0; kc < nk; ++kc) {
+      if (layer > 0 && !chain_wait(sm, &sm->written[kc], (layer - 1) & 1)) return false;
+      const uint64_t da = act_desc + (uint64_t)((kc % kActSpans) * (kSpanBytes >> 4));
+      for (int half = 0; half < halves; ++half) {
+        if (!chain_wait(sm, &sm->full[slot], ph)) return false;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint64_t db = ring_desc + (uint64_t)(slot * (kSpanBytes >> 4));
+#pragma unroll
+        for (int ks = 0; ks < kChunkK / 16; ++ks)
+          mma_bf16(sums + half * kPieceN, da + 2 * ks, db + 2 * ks, idesc, kc != 0 || ks != 0);
+        mma_commit(smem_u32(&sm->empty[slot]));
+        if (++slot == kRing) {
+          slot = 0;
+          ph ^= 1;
+        }
+      }
+    }
+    mma_commit(smem_u32(&sm->done));
+  }
+  return true;
+}
+
+__global__ void __launch_bounds__(kChainThreads, 1) chain_kernel(const __grid_constant__ Chain c) {
+  extern __shared__ __align__(1024) unsigned char dsmem[];
+  unsigned char* act = dsmem;
+  unsigned char* ring = dsmem + kActSpans * kSpanBytes;
+  ChainBars* sm = reinterpret_cast<ChainBars*>(ring + kRing * kSpanBytes);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m0 = blockIdx.x * kTileM;
+  if (smem_u32(dsmem) & 1023) {  // the swizzled spans want what the declaration asks for
+    if (threadIdx.x == 0 && c.error) atomicExch(c.error, 3);
+    return;
+  }
+
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" : : "r"(smem_u32(&sm->tmem_base)), "r"(2 * kChainWidth));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (threadIdx.x == 0) {
+    const auto init = [](const uint64_t* bar, int count) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" : : "r"(smem_u32(bar)), "r"(count));
+    };
+    for (int s = 0; s < kRing; ++s) {
+      init(&sm->full[s], 1);
+      init(&sm->empty[s], 1);
+    }
+    for (int s = 0; s < kActSpans; ++s) init(&sm->written[s], kEpiWarps);
+    init(&sm->done, 1);
+    init(&sm->drained, 1);
+    sm->failed = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = sm->tmem_base;
+
+  const int nk0 = (c.nin + kChunkK - 1) / kChunkK;
+  if (warp == kEpiWarps) {
+    int copied = 0;
+    if (lane == 0 && !chain_copy(c, sm, smem_u32(act), smem_u32(ring), m0, nk0, &copied)) {
+      // the copies in flight end before the shared memory goes
+      for (int p = copied > kRing ? copied - kRing : 0; p < copied; ++p)
+        mbar_wait(smem_u32(&sm->full[p % kRing]), (p / kRing) & 1);
+    }
+    __syncwarp();
+  } else if (warp == kEpiWarps + 1) {
+    if (lane == 0 && !chain_multiply(sm, smem_u32(act), smem_u32(ring), tmem, nk0)) {
+      mma_commit(smem_u32(&sm->drained));  // and so do the products
+      mbar_wait(smem_u32(&sm->drained), 0);
+    }
+    __syncwarp();
+  } else {
+    // lane = row; a warp takes kBlockN columns of each span
+    const int quad = warp & 3, part = warp >> 2, row = 32 * quad + lane;
+    const uint32_t tmem_row = tmem + ((uint32_t)(32 * quad) << 16);
+    bool good = true;
+    for (int layer = 0; layer < kChainLayers; ++layer) {
+      good = __all_sync(0xffffffffu, chain_wait(sm, &sm->done, layer & 1));
+      if (!good) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t sums = tmem_row + (layer & 1) * kChainWidth;
+      if (layer < kChainLayers - 1) {
+        for (int span = 0; span < kActSpans; ++span) {
+          float v[kBlockN];
+          tmem_ld16(sums + (uint32_t)(span * kSpan + part * kBlockN), v);
+          const float* b = c.bias[layer] + span * kSpan + part * kBlockN;
+          const bool vec = (reinterpret_cast<uintptr_t>(b) & 15) == 0;  // the parameters may lie anywhere
+          unsigned char* dst = act + span * kSpanBytes + row * 128;
+#pragma unroll
+          for (int q = 0; q < kBlockN / 8; ++q) {
+            const float4 b0 = bias4(b + 8 * q, vec), b1 = bias4(b + 8 * q + 4, vec);
+            uint4 h;
+            h.x = pack_bf16(gelu(v[8 * q] + b0.x), gelu(v[8 * q + 1] + b0.y));
+            h.y = pack_bf16(gelu(v[8 * q + 2] + b0.z), gelu(v[8 * q + 3] + b0.w));
+            h.z = pack_bf16(gelu(v[8 * q + 4] + b1.x), gelu(v[8 * q + 5] + b1.y));
+            h.w = pack_bf16(gelu(v[8 * q + 6] + b1.z), gelu(v[8 * q + 7] + b1.w));
+            *reinterpret_cast<uint4*>(dst + (((part * kBlockN / 8 + q) ^ (row & 7)) << 4)) = h;
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads what was written here
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0)
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" : : "r"(smem_u32(&sm->written[span])) : "memory");
+        }
+      } else if (part == 0) {
+        // the outputs: through a padded block of the (now unused) activations to whole lines
+        float* tf = reinterpret_cast<float*>(act) + warp * 32 * 33;
+        const float* b = c.bias[layer];
+        for (int c0 = 0; c0 < kChainOut; c0 += kBlockN) {
+          float v[kBlockN];
+          tmem_ld16(sums + (uint32_t)c0, v);
+#pragma unroll
+          for (int j = 0; j < kBlockN; ++j) tf[lane * 33 + c0 + j] = v[j] + __ldg(b + c0 + j);
+        }
+        __syncwarp();
+        for (int r = 0; r < 32; ++r) {
+          const int grow = m0 + 32 * quad + r;
+          if (grow < c.rows) c.out[(size_t)grow * kChainOut + lane] = tf[r * 33 + lane];
+        }
+      }
+    }
+    if (!good && lane == 0 && c.error) atomicExch(c.error, 1);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" : : "r"(tmem), "r"(2 * kChainWidth));
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -438,11 +699,11 @@ int choose_ntile(int M, int N) {
   return nt;
 }
 
-// The kernel's dynamic shared-memory limit is raised once per device to what the largest ring
+// The kernels' dynamic shared-memory limits are raised once per device, gemm_kernel's to what the largest ring
 // needs, and never lowered: a launch with a smaller one needs less, and a CUDA graph whose nodes were
 // captured with different tile widths stays launchable whatever was set last.
 constexpr int kMaxDevices = 64;
-cudaError_t set_smem_limit_once() {
+cudaError_t set_smem_limits_once() {
   static std::mutex mu;
   static uint64_t done_ctx[kMaxDevices] = {0};  // context_id() the limit was set in (0: not set)
   int dev = 0;
@@ -456,6 +717,8 @@ cudaError_t set_smem_limit_once() {
   if (smem_bytes(128, 3) > most) most = smem_bytes(128, 3);
   if (smem_bytes(64, kMaxStages) > most) most = smem_bytes(64, kMaxStages);
   e = cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmem);
   if (e == cudaSuccess) done_ctx[dev] = context_id();
   return e;
 }
@@ -507,9 +770,37 @@ cudaError_t launch(const GemmOperands* op, const GemmArgs* g, int problems, cuda
   b.first[problems] = (int)blocks;
   b.n = problems;
   b.stages = choose_stages(nt, chunks);
-  const cudaError_t attr = set_smem_limit_once();
+  const cudaError_t attr = set_smem_limits_once();
   if (attr != cudaSuccess) return attr;
   gemm_kernel<<<(unsigned)blocks, kThreads, smem_bytes(nt, b.stages), s>>>(b);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_chain(const ChainOperands& op, int rows, int nin, int* error, cudaStream_t s, const char** why) {
+  *why = nullptr;
+  Chain c;
+  c.out = op.out;
+  c.error = error;
+  c.rows = rows;
+  c.nin = nin;
+  if (rows < 1 || nin < 1 || nin % 8) *why = "GEMM contiguous extents must be multiples of 8";
+  if (((uintptr_t)op.x | (uintptr_t)op.w[0]) & 15) *why = "GEMM operands must be 16-byte aligned";
+  if (nin > (1 << 24)) *why = "GEMM too large";
+  if (*why) return cudaErrorInvalidValue;
+  bool ok = make_map(&c.x, op.x, rows, nin, nin, kTileM);
+  for (int l = 0; l < kChainLayers; ++l) {
+    const bool last = l == kChainLayers - 1;
+    const int k = l == 0 ? nin : kChainWidth, n = last ? kChainOut : kChainWidth;
+    ok = ok && make_map(&c.w[l], op.w[l], n, k, k, last ? kChainOut : kPieceN);
+    c.bias[l] = op.bias[l];
+  }
+  if (!ok) {
+    *why = "cuTensorMapEncodeTiled failed (driver entry point missing or unsupported tensor shape)";
+    return cudaErrorInvalidValue;
+  }
+  const cudaError_t attr = set_smem_limits_once();
+  if (attr != cudaSuccess) return attr;
+  chain_kernel<<<(unsigned)(((long long)rows + kTileM - 1) / kTileM), kChainThreads, kChainSmem, s>>>(c);
   return cudaGetLastError();
 }
 

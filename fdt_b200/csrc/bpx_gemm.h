@@ -46,5 +46,18 @@ int choose_ntile(int M, int N);
 // Validates the arguments (why = reason on failure) and launches on stream s.
 cudaError_t launch(const GemmOperands* op, const GemmArgs* g, int problems, cudaStream_t s, const char** why);
 
+// The network's layers: kChainLayers - 1 of kChainWidth outputs with bias and GELU, then kChainOut with bias.
+constexpr int kChainWidth = 256, kChainLayers = 5, kChainOut = 32;
+
+struct ChainOperands {
+  const uint16_t* x;                // bf16 [rows][nin]
+  const uint16_t* w[kChainLayers];  // bf16 [outputs][inputs]
+  const float* bias[kChainLayers];
+  float* out;  // [rows][kChainOut]
+};
+
+// All layers in one launch, nothing but the last one's outputs written.
+cudaError_t launch_chain(const ChainOperands& op, int rows, int nin, int* error, cudaStream_t s, const char** why);
+
 }  // namespace gemm
 }  // namespace bpx

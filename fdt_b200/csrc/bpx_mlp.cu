@@ -42,7 +42,6 @@ constexpr int kOutProps = 17;  // first proposal-width output
 // is near zero without bound (every proposal is accepted; CUDA/runmcmc_kernels.cu caps them at
 // 1e10), but a width past e^2 (> 2 pi for an angle, > 1 for a fraction) proposes no differently.
 constexpr float kLogWidthMin = -14.f, kLogWidthMax = 2.f;
-constexpr int kMaxChunk = 32768;  // inference rows per pass (bounds the activation buffers)
 
 struct Geom {
   int nin;
@@ -452,22 +451,43 @@ bpx_status cast_weights(const Geom& G, const float* params, uint16_t* wbf, float
   return BPX_OK;
 }
 
-// forward pass of rows [0, n) of x; activations in the network workspace
-bpx_status forward(const Geom& G, const float* params, const uint16_t* wbf, int n, const uint16_t* x, float* out,
-                   uint16_t* buf0, uint16_t* buf1, float* const* z, uint16_t* const* acts, int* err, cudaStream_t s) {
+// forward pass that keeps each layer's sums z and activations for the backward pass
+bpx_status forward_keep(const Geom& G, const float* params, const uint16_t* wbf, int n, const uint16_t* x, float* out,
+                        float* const* z, uint16_t* const* acts, int* err, cudaStream_t s) {
   const uint16_t* a = x;
   int lda = G.nin;
   for (int l = 0; l < kLayers - 1; ++l) {
-    uint16_t* o = acts ? acts[l] : ((l & 1) ? buf1 : buf0);
-    bpx_status st = run_gemm(a, lda, 0, wbf + G.wbf[l], G.k[l], 0, n, G.n[l], G.k[l], gemm::kEpiBiasGelu,
-                             z ? z[l] : nullptr, G.n[l], o, G.n[l], params + G.boff[l], nullptr, 0, err, s);
+    bpx_status st = run_gemm(a, lda, 0, wbf + G.wbf[l], G.k[l], 0, n, G.n[l], G.k[l], gemm::kEpiBiasGelu, z[l], G.n[l],
+                             acts[l], G.n[l], params + G.boff[l], nullptr, 0, err, s);
     if (st != BPX_OK) return st;
-    a = o;
+    a = acts[l];
     lda = G.n[l];
   }
   const int l = kLayers - 1;
   return run_gemm(a, lda, 0, wbf + G.wbf[l], G.k[l], 0, n, G.n[l], G.k[l], gemm::kEpiBias, out, kOut, nullptr, 0,
                   params + G.boff[l], nullptr, 0, err, s);
+}
+
+static_assert(kWidth == gemm::kChainWidth && kLayers == gemm::kChainLayers && kOut == gemm::kChainOut, "the chain's shape");
+
+// forward pass for its outputs alone, wbf receiving the BF16 weights
+bpx_status infer(const Geom& G, const float* params, uint16_t* wbf, int n, const uint16_t* x, float* out, cudaStream_t s) {
+  int* err = nullptr;
+  bpx_status st = error_word(&err);
+  if (st == BPX_OK) st = cast_weights(G, params, wbf, nullptr, s);
+  if (st != BPX_OK) return st;
+  gemm::ChainOperands op{};
+  op.x = x;
+  op.out = out;
+  for (int l = 0; l < kLayers; ++l) {
+    op.w[l] = wbf + G.wbf[l];
+    op.bias[l] = params + G.boff[l];
+  }
+  const char* why = nullptr;
+  const cudaError_t e = gemm::launch_chain(op, n, G.nin, err, s, &why);
+  if (why) return api_fail(BPX_ERR_INVALID_ARG, std::string("tcgen05 GEMM: ") + why);
+  if (e != cudaSuccess) return api_cuda_fail(e, "network launch");
+  return BPX_OK;
 }
 
 Layout layout_of(const bpx_options* o) {
@@ -488,18 +508,9 @@ namespace bpx {
 size_t mlp_weight_elems(int ndir) { return geom(ndir).nw; }
 
 bpx_status mlp_forward_buffers(int ndir, const float* params, int nvox, const uint16_t* x, float* out, uint16_t* wbf,
-                               uint16_t* buf0, uint16_t* buf1, int chunk_rows, cudaStream_t s) {
+                               cudaStream_t s) {
   NvtxRange nvtx_range("bpx.network");
-  const Geom G = geom(ndir);
-  int* err = nullptr;
-  bpx_status st = error_word(&err);
-  if (st == BPX_OK) st = cast_weights(G, params, wbf, nullptr, s);
-  for (int r0 = 0; st == BPX_OK && r0 < nvox; r0 += chunk_rows) {
-    const int n = std::min(chunk_rows, nvox - r0);
-    st = forward(G, params, wbf, n, x + (size_t)r0 * G.nin, out + (size_t)r0 * kOut, buf0, buf1, nullptr, nullptr, err,
-                 s);
-  }
-  return st;
+  return nvox > 0 ? infer(geom(ndir), params, wbf, nvox, x, out, s) : BPX_OK;
 }
 
 }  // namespace bpx
@@ -558,28 +569,10 @@ bpx_status bpx_mlp_forward_dev(int32_t ndir, const float* params, int32_t nvox, 
   bpx_status st = api_check_device();
   if (st != BPX_OK) return st;
   const Geom G = geom(ndir);
-  const int chunk = std::min<int>(nvox, kMaxChunk);
-  const size_t b_w = a256(G.nw * 2), b_act = a256((size_t)chunk * kWidth * 2);
   void* ws = nullptr;
-  st = api_workspace(kWsNetwork, b_w + 2 * b_act, &ws);
+  st = api_workspace(kWsNetwork, a256(G.nw * 2), &ws);
   if (st != BPX_OK) return st;
-  int* err = nullptr;
-  st = error_word(&err);
-  if (st != BPX_OK) return st;
-  char* p = (char*)ws;
-  uint16_t* wbf = (uint16_t*)p;
-  uint16_t* buf0 = (uint16_t*)(p + b_w);
-  uint16_t* buf1 = (uint16_t*)(p + b_w + b_act);
-  cudaStream_t s = (cudaStream_t)stream;
-  st = cast_weights(G, params, wbf, nullptr, s);
-  if (st != BPX_OK) return st;
-  for (int r0 = 0; r0 < nvox; r0 += chunk) {
-    const int n = std::min(chunk, nvox - r0);
-    st = forward(G, params, wbf, n, x + (size_t)r0 * G.nin, out + (size_t)r0 * kOut, buf0, buf1, nullptr, nullptr,
-                 err, s);
-    if (st != BPX_OK) return st;
-  }
-  return BPX_OK;
+  return infer(G, params, (uint16_t*)ws, nvox, x, out, (cudaStream_t)stream);
 }
 
 bpx_status bpx_mlp_train_step_dev(int32_t ndir, const float* params, float* grads, int32_t batch, const uint16_t* x,
@@ -621,7 +614,7 @@ bpx_status bpx_mlp_train_step_dev(int32_t ndir, const float* params, float* grad
   cudaStream_t s = (cudaStream_t)stream;
   st = cast_weights(G, params, wbf, loss, s);
   if (st != BPX_OK) return st;
-  st = forward(G, params, wbf, batch, x, out, nullptr, nullptr, z, acts, err, s);
+  st = forward_keep(G, params, wbf, batch, x, out, z, acts, err, s);
   if (st != BPX_OK) return st;
   loss_kernel<<<(batch + kLossRows - 1) / kLossRows, 256, 0, s>>>(batch, out, targets, tweights, dz[kLayers - 1], loss);
   MLP_CUDA(cudaGetLastError());

@@ -171,6 +171,47 @@ def test_gemm_at_the_edges_of_its_spans(torch, M, N, K, a_mn, b_mn):
     assert bool(((c.cpu().double() - ref).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("rows", [1, 127, 128, 129, 700])
+@pytest.mark.parametrize("ndir", [1, 64, 65, 256, 257, 330, 700])
+def test_inference_at_the_edges_of_its_tiles(torch, rows, ndir):
+    """All layers run in one launch, 128 rows to a block, the inputs in chunks of 64 of which four are held
+    at a time.  Against the NumPy oracle within 1e-2 (activations rounded to BF16 per layer); bit for bit
+    the same for any number of rows, and for parameters and outputs at any 4-byte address."""
+    import ctypes as C
+
+    from fdt_b200 import learned, lib
+    from oracle import mlp_oracle as M
+
+    rng = np.random.default_rng(rows + ndir)
+    p = learned.init_params(ndir, 3)
+    k, n, _, boff, _ = learned.geometry(ndir)
+    for l in range(5):
+        p[boff[l]:boff[l] + n[l]] = 0.05 * rng.normal(size=n[l])
+    nin = (ndir + 7) // 8 * 8
+    x = np.zeros((rows, nin), np.float32)
+    x[:, :ndir] = np.exp(-rng.uniform(0.0, 2.0, (rows, ndir)))
+    xd = torch.from_numpy(x).to(torch.bfloat16).cuda()
+    xq = xd.float().cpu().numpy()
+
+    def run(n, shift):
+        pd = torch.zeros(p.size + shift, device="cuda")
+        pd[shift:] = torch.from_numpy(p).cuda()
+        out = torch.full((n * 32 + shift + 32,), -7.0, device="cuda")
+        rc = lib.load().bpx_mlp_forward_dev(ndir, pd.data_ptr() + 4 * shift, n, xd.data_ptr(), out.data_ptr() + 4 * shift,
+                                            C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert rc == 0
+        torch.cuda.synchronize()
+        assert lib.poll_error() == 0
+        assert bool((out[:shift] == -7.0).all()) and bool((out[shift + n * 32:] == -7.0).all())
+        return out[shift:shift + n * 32].reshape(n, 32).cpu().numpy()
+
+    out = run(rows, 0)
+    ref, _ = M.forward(p, ndir, xq)
+    assert np.linalg.norm(out - ref) < 1e-2 * np.linalg.norm(ref)
+    assert np.array_equal(out, run(rows, 1))
+    assert np.array_equal(out[:(rows + 1) // 2], run((rows + 1) // 2, 0))
+
+
 @pytest.mark.parametrize("batch", [1, 63, 65, 960, 961, 2049])
 def test_gradients_at_the_edges_of_the_batch_split(torch, batch):
     """From 16 chunks of 64 rows (961 rows) the weight gradients' contractions run in two parts.  The bounds
