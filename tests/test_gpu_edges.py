@@ -271,3 +271,21 @@ def test_tracking_small_calls_equal_oracle(torch, nparticles, kw):
     assert np.array_equal(got[0].cpu().numpy(), want[0]) and got[1] == want[1]
     if targets is not None:
         assert np.array_equal(got[2], want[2])
+
+
+@pytest.mark.parametrize("nfibres", [1, 2, 3])
+@pytest.mark.parametrize("nsamples", [1, 31, 32, 33, 50])
+@pytest.mark.parametrize("shape", [(37, 12, 9), (16, 8, 8)])
+def test_tracking_equals_oracle_for_any_sample_count(torch, nfibres, nsamples, shape):
+    """The samples are repacked in tiles of 32 voxels by 32 samples, by a kernel per fibre count: counts below,
+    at and past whole tiles, with and without a partial tile of voxels; a fibre without a direction."""
+    from fdt_b200 import lib
+
+    th, ph, f, mask = synth.fibre_field(shape, nsamples=nsamples, seed=nsamples)
+    th, ph, f = (np.ascontiguousarray(np.concatenate([q] * 3)[:nfibres]) for q in (th, ph, f))
+    th[-1, :, :, :, ::5] = 0.0
+    o = TrackOptions.make(nparticles=200, nsteps=300, seed=3, randfib=1)
+    seeds = np.array([[shape[0] // 2, shape[1] // 2, shape[2] // 2]], np.float32)
+    got = lib.probtrack(o, *(lib.to_device(q) for q in (th, ph, f, mask)), seeds)
+    want = O.probtrack(o, th, ph, f, mask, seeds)
+    assert np.array_equal(got[0].cpu().numpy(), want[0]) and got[1] == want[1]
