@@ -812,13 +812,10 @@ def main():
 
     steps_fn = {"plain": plain_step, "learned": learned_step, "learned_batched": learned_batched_step,
                 "lm_burnin200": lm200_step}
-    # learned: prepare, features, weight cast + 5 GEMMs per 32768 voxels, decode, mcmc, finish;
-    # learned_batched: one CUDA-graph launch (gather, the same kernels, scatter)
-    n_gemm = 5 * ((chunk + 32767) // 32768)
     # kernels per step: plain = Rician clean-up, 4 fit stages, MCMC, finishing; learned = clean-up,
-    # features, weight cast, the GEMMs, decode, MCMC, finishing; the graph form launches once and its
+    # features, weight cast, the network, decode, MCMC, finishing; the graph form launches once and its
     # graph holds gather, the learned form's kernels and scatter
-    launches = {"plain": 7, "learned": 6 + n_gemm, "learned_batched": 8 + n_gemm, "lm_burnin200": 7}
+    launches = {"plain": 7, "learned": 7, "learned_batched": 9, "lm_burnin200": 7}
     timing = {}
     clocks = ClockSampler(local)
     clocks.start()

@@ -6,8 +6,9 @@
 //
 // Network: x (ndir signals / S0_hat, padded to nin = 8*ceil(ndir/8)) -> 256 -> 256 -> 256 -> 256
 // (GELU after each) -> 32 outputs.  BF16 weights and activations, FP32 accumulation, FP32 master
-// parameters.  Every contraction (forward, dX, dW) runs on the tcgen05 GEMM of bpx_gemm.cu with
-// the bias, GELU and GELU-derivative fused into its epilogue.
+// parameters.  Every contraction runs on the tcgen05 kernels of bpx_gemm.cu with the bias, GELU and
+// GELU-derivative fused into their epilogues: inference as one launch for all layers, training (forward
+// with the sums kept, dX, dW) layer by layer.
 //
 // Flat parameter vector (FP32): for layer l = 0..4, W_l [n_l][k_l] row-major then b_l [n_l];
 // k = {nin, 256, 256, 256, 256}, n = {256, 256, 256, 256, 32}.
@@ -587,7 +588,7 @@ bpx_status bpx_mlp_train_step_dev(int32_t ndir, const float* params, float* grad
   const size_t b_out = a256(B * kOut * 4), b_dz5 = a256(B * kOut * 2);
   // the weight gradients' outputs are a few tiles each with the whole batch to contract: 32-column
   // tiles of all layers in one launch, each contraction in two parts, give every SM a CTA at 4096
-  // rows.  (Eight parts are no faster end to end, 165 us a step either way, and move the sums, whose
+  // rows.  (Eight parts are no faster end to end and move the sums, whose
   // accumulation the tensor core rounds, nearer to 1e-5 from the undivided ones.)
   const int chunks = (batch + 63) / 64;
   const int splits = chunks >= 16 ? 2 : 1;

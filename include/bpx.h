@@ -532,9 +532,11 @@ void bpx_track_options_default(bpx_track_options* opts);
  * the kept streamlines to *waytotal (device int64); the caller zeroes both first.  Integer sums make the result independent of the order in which streamlines finish.
  * Uses workspace memory (see Concurrency): the samples repacked, 16 * (nfib + 1) bytes per voxel
  * and sample, and per particle in flight a visit table of 8 * 2^ceil(log2(2 * (nsteps + 2))) bytes
- * (twice that with matrix2) and with loopcheck a coarse-cell table of 24 bytes per entry; 1024
- * particles in flight per multiprocessor, fewer if the tables would pass 16 GB (5 GB on a B200 at
- * nsteps 2000 without options).
+ * (twice that with matrix2), with loopcheck a coarse-cell table of 24 bytes per entry, and with avoid,
+ * waypoints or distthresh lists of 4 * nsteps bytes (not where those options track particles twice: with
+ * matrix2, or targets and distthresh); 1024 particles in flight per multiprocessor, or the call's own
+ * number if that is less, fewer if all this would pass 16 GB (5 GB on a B200 at nsteps 2000 without
+ * options).
  */
 bpx_status bpx_probtrack_dev(const bpx_track_options* opts, const bpx_track_volume* vol, int32_t nseeds,
                              const float* seeds, int32_t* paths, int64_t* waytotal, void* stream);
