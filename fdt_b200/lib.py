@@ -385,15 +385,20 @@ def waypoint_bits(masks) -> np.ndarray:
     masks = list(masks)
     if not 1 <= len(masks) <= 32:
         raise ValueError("1 to 32 waypoint masks")
-    # eight masks at a time in a byte, widened once: a third of the time of widening every mask
+    # eight masks at a time in a byte, widened once: a third of the time of widening every mask.  The first
+    # mask gives the shape, to which all others are broadcast, in whatever group of eight they are
     bits = None
     for first in range(0, len(masks), 8):
-        byte = (np.asarray(masks[first]) != 0).view(np.uint8)
+        byte = np.empty(np.shape(masks[0]), np.uint8)
+        np.not_equal(np.asarray(masks[first]), 0, out=byte.view(np.bool_))
         for w, m in enumerate(masks[first + 1 : first + 8], 1):
             byte |= (np.asarray(m) != 0).view(np.uint8) << np.uint8(w)
         wide = byte.astype(np.uint32)
-        bits = wide if bits is None else bits | (wide << np.uint32(first))
-    return np.ascontiguousarray(bits).view(np.int32)
+        if bits is None:
+            bits = wide
+        else:
+            bits |= wide << np.uint32(first)
+    return bits.view(np.int32)
 
 
 def matrix2_lookup(lrmask) -> np.ndarray:
