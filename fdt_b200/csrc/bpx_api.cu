@@ -35,7 +35,6 @@ int g_sm_count[kMaxDevices] = {0};
 // compiled (tpv, mpl) layouts, in order of preference for a given capacity
 const McmcLayout kLayouts[] = {{4, 9}, {8, 8}, {8, 9}, {16, 9}, {32, 9}, {32, 16}};
 constexpr int kNumLayouts = sizeof(kLayouts) / sizeof(kLayouts[0]);
-constexpr int kMaxNdir = 512;
 
 bpx_status fail(bpx_status st, const std::string& msg) {
   g_last_error = msg;

@@ -1240,12 +1240,15 @@ __global__ void __launch_bounds__(kFitThreads) prepare_kernel(int nvox, int ndir
 // ------------------------------------------------------------------------------------------
 // launchers
 // ------------------------------------------------------------------------------------------
-// One stage over every voxel: as many blocks as fit the device at once, fewer for small volumes.
+// One stage over every voxel: as many blocks as fit the device at once, fewer for small volumes.  The limit
+// on a kernel's dynamic shared memory belongs to the process, not to the call: it is only ever set to
+// smem_most, the need at kMaxNdir, so that no call lowers it between another thread's setting and launch, or
+// below what a captured launch needs.
 static cudaError_t launch_stage(void (*kern)(FitArgs, unsigned int*), const FitArgs& a, unsigned int* queue, size_t smem,
-                                cudaStream_t s) {
+                                size_t smem_most, cudaStream_t s) {
   int per_sm = 0;
   cudaError_t e = cudaSuccess;
-  if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_most);
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFitThreads, smem);
   if (e != cudaSuccess) return e;
   const int cap = sm_count() * (per_sm > 0 ? per_sm : 1), warps = kFitThreads / 32;
@@ -1260,11 +1263,11 @@ static cudaError_t launch_fit_kf(const FitArgs& a, cudaStream_t s) {
   static_assert(LmShape<kMulti, K, F0>::P <= 14, "scratch doubles 14 and 15 hold the voxel counters");
   unsigned int* queue = reinterpret_cast<unsigned int*>(a.scratch + 14);
   cudaError_t e = cudaMemsetAsync(queue, 0, 4 * sizeof(unsigned int), s);
-  const size_t smem = single_block_bytes(a.ndir) + (kFitThreads / 32) * single_warp_bytes(K, a.ndir);
-  if (e == cudaSuccess) e = launch_stage(fit_start_kernel<K, F0>, a, queue, smem, s);
-  if (e == cudaSuccess && a.model >= 2) e = launch_stage(fit_multi_kernel<K, F0>, a, queue + 1, 0, s);
-  if (e == cudaSuccess && F0) e = launch_stage(fit_refit_kernel<K>, a, queue + 2, 0, s);
-  if (e == cudaSuccess) e = launch_stage(fit_finish_kernel<K, F0>, a, queue + 3, 0, s);
+  const auto need = [](int ndir) { return single_block_bytes(ndir) + (kFitThreads / 32) * single_warp_bytes(K, ndir); };
+  if (e == cudaSuccess) e = launch_stage(fit_start_kernel<K, F0>, a, queue, need(a.ndir), need(kMaxNdir), s);
+  if (e == cudaSuccess && a.model >= 2) e = launch_stage(fit_multi_kernel<K, F0>, a, queue + 1, 0, 0, s);
+  if (e == cudaSuccess && F0) e = launch_stage(fit_refit_kernel<K>, a, queue + 2, 0, 0, s);
+  if (e == cudaSuccess) e = launch_stage(fit_finish_kernel<K, F0>, a, queue + 3, 0, 0, s);
   return e;
 }
 

@@ -19,6 +19,7 @@ struct NvtxRange {
   NvtxRange& operator=(const NvtxRange&) = delete;
 };
 
+constexpr int kMaxNdir = 512;      // measurements of a voxel
 constexpr int kFitThreads = 128;   // 4 warps, one voxel per warp at a time
 #ifndef BPX_FIT_MIN_BLOCKS
 #define BPX_FIT_MIN_BLOCKS 4
