@@ -10,7 +10,8 @@
 // waypoint masks or a distance threshold, which halves are kept is known only when both have ended:
 // the halves' voxels are listed as they are tracked and the kept lists counted afterwards (with
 // --omatrix2, or targets under a distance threshold, whose counts need the positions or path lengths
-// along the way, the kept halves are tracked again: the same draws, so the same path).
+// along the way, and where the tables of very long paths leave few particles in flight, the kept halves are
+// tracked again: the same draws, so the same path).
 //
 // The work is a chain of dependent random gathers (the mask at the position and a posterior sample
 // at a randomly rounded position, then the step), so the kernel is latency-bound: a persistent
@@ -299,7 +300,7 @@ struct Tracker {
     }
   }
 
-  // counts a kept half from its list of voxels, as half_line counts while it tracks (targets without a
+  // counts a kept half from its list of voxels, as step() counts while it tracks (targets without a
   // distance threshold: every entry's path is long enough)
   template <int FEAT>
   __device__ void count_list(const uint32_t* list, int n, int& nvisit, Counted& cnt) const {
@@ -497,7 +498,7 @@ struct Tracker {
     load_record(svox, samp, S);
     if (!(in_grid && m > 0.f)) return false;  // the reference's remaining steps change nothing
     if ((FEAT & kFeatLoop) && o.loopcheck) {
-      // stop where the path runs against the direction it H.last had in this coarse cell
+      // stop where the path runs against the direction it last had in this coarse cell
       const int lx = lc_round(P.x), ly = lc_round(P.y), lz = lc_round(P.z);
       const uint32_t cell = ((uint32_t)lz * (uint32_t)a.lcny + (uint32_t)ly) * (uint32_t)a.lcnx + (uint32_t)lx;
       float3 old = H.lc_dir;
@@ -607,11 +608,11 @@ struct Tracker {
 // Every thread walks its particles (pid_begin + thread, then one grid further each time), both halves of
 // each.  The halves of a warp's lanes end at different steps, so the steps are the warp's one loop and
 // a lane whose half has ended begins its next one there, instead of waiting for the warp's longest
-// (512 seeds x 5000 particles: 21.2 -> 17.3 ms).  With kFeatKeep an ended half can lead to counting its
-// list, which is long for one lane alone: the warp then waits until kRefillKeep lanes have ended
+// (512 seeds x 5000 particles: 21.2 -> 17.3 ms).  With lists an ended half can lead to counting its
+// list, which is long for one lane alone: the warp then waits until kRefillLists lanes have ended
 // (distthresh on that field, 128 seeds: 10.8 ms with 1, 9.1 ms with 8; without lists 8 cost 26 ms
-// against 17.5: the lanes that wait are then the loss).
-constexpr int kRefillKeep = 8;
+// against 17.5, and where halves are tracked twice 9.6 against 8.9: the lanes that wait are then the loss).
+constexpr int kRefillLists = 8;
 
 template <int FEAT>
 __global__ void __launch_bounds__(kTrackThreads, kTrackBlocksPerSm) track_kernel(TrackArgs a) {
@@ -624,6 +625,7 @@ __global__ void __launch_bounds__(kTrackThreads, kTrackBlocksPerSm) track_kernel
   }
   unsigned long long kept = 0;
   uint32_t* const list0 = (FEAT & kFeatKeep) && a.lists ? a.lists + t * 2 * a.list_cap : nullptr;
+  const int refill = list0 ? kRefillLists : 1;
   uint64_t pid = a.pid_begin + t;
   Particle P{};
   Tracker::Half H{};
@@ -638,7 +640,7 @@ __global__ void __launch_bounds__(kTrackThreads, kTrackBlocksPerSm) track_kernel
   for (;;) {
     const unsigned running = __ballot_sync(0xffffffffu, active), waiting = __ballot_sync(0xffffffffu, !active && more);
     if (!(running | waiting)) break;
-    if (__popc(waiting) >= ((FEAT & kFeatKeep) ? kRefillKeep : 1) || !running) {
+    if (__popc(waiting) >= ((FEAT & kFeatKeep) ? refill : 1) || !running) {
       if (!active && more) {
         // what the ended half leads to
         if (FEAT & kFeatKeep) {
@@ -941,21 +943,34 @@ bpx_status bpx_probtrack_dev(const bpx_track_options* opts, const bpx_track_volu
   // would pass 16 GB
   const size_t table_bytes = ((size_t)1 << log2n) * sizeof(uint2);
   const bool keep = opts->distthresh > 0.f || vol->avoid != nullptr || vol->nwaypoints > 0;
-  // the lists of a particle's voxels, one per half with an entry per step at most; the counts that need
-  // more than the voxels are made by tracking the kept halves again
-  const bool list = keep && vol->m2_ncols == 0 && (vol->ntargets == 0 || !(opts->distthresh > 0.f));
+  const uint64_t total = (uint64_t)nseeds * (uint64_t)opts->nparticles;
+  const uint64_t want = (total + kTrackThreads - 1) / kTrackThreads;
+  const auto blocks_within = [&](size_t list) { return ((size_t)16 << 30) / ((table_bytes + lc_bytes + list) * kTrackThreads); };
+  // The lists of a particle's voxels, one per half with an entry per step at most.  The counts that need more
+  // than the voxels are made by tracking the kept halves again.  So are all where the tables of long paths
+  // leave the lists under half of the resident blocks and of the blocks the call could use: the lists take a
+  // share of what is left, and nothing hides their counting's chains of loads.  (Paths of 2000, 8100, 10000,
+  // 20000 and 40000 steps at most, 64 seeds x 8000 particles, a waypoint, 1 fibre: lists 5.1, 7.2, 10.2,
+  // 17.0, 30.5 ms, twice 5.2, 7.0, 8.9, 13.2, 21.1 ms; 3 fibres: 6.3, 8.0, 11.9, 18.4, 32.7 and 6.3, 8.3,
+  // 10.1, 15.0, 24.3 ms.  64 x 1000, an avoid mask, 2 fibres, 16000 and 40000 steps: 3.0, 4.2 and 3.4, 4.0.)
+  // The second tracking costs a path's steps, the lists its voxels: with 20 steps across a voxel, 64 x 1000,
+  // 20000 steps and 1, 2, 3 fibres the lists took 9.4, 11.4, 10.8 ms and twice 8.6, 10.5, 11.9; with 40, 40000
+  // steps 19.7, 22.8, 24.1 and 22.1, 23.7, 30.0 ms; from 20 on the lists stay.  They do with loopcheck,
+  // whose tables a second tracking would use again (10000 steps, 64 x 8000, 2 fibres: 19.3 and 22.5 ms).
   a.list_cap = (size_t)(opts->nsteps / 2);
-  const size_t list_bytes = list ? 2 * a.list_cap * sizeof(uint32_t) : 0;
-  const size_t max_blocks = ((size_t)16 << 30) / ((table_bytes + lc_bytes + list_bytes) * kTrackThreads);
+  const size_t half_lists = 2 * a.list_cap * sizeof(uint32_t), list_blocks = blocks_within(half_lists);
+  const bool roomy = list_blocks >= (size_t)sm_count() * kTrackBlocksPerSm / 2 || 2 * list_blocks >= want;
+  const bool list = keep && vol->m2_ncols == 0 && (vol->ntargets == 0 || !(opts->distthresh > 0.f)) &&
+                    (roomy || opts->loopcheck || dmin >= 20.f * opts->steplength);
+  const size_t list_bytes = list ? half_lists : 0;
+  const size_t max_blocks = blocks_within(list_bytes);
   const int feat = (opts->modeuler ? kFeatEuler : 0) | (opts->loopcheck ? kFeatLoop : 0) |
                    ((vol->ntargets > 0 || vol->m2_ncols > 0 || vol->m1_ncols > 0) ? kFeatCount : 0) |
                    (vol->prefdir ? kFeatPref : 0) | (keep ? kFeatKeep : 0);
-  const uint64_t total = (uint64_t)nseeds * (uint64_t)opts->nparticles;
   int grid = sm_count() * kTrackBlocksPerSm;
   if ((size_t)grid > max_blocks) grid = max_blocks > 0 ? (int)max_blocks : 1;
   // no more threads than particles: the tables, which are cleared for every call, shrink with the call
   // (4 seeds x 5000 particles: 0.7 ms of clearing 5 GB against 0.1 ms)
-  const uint64_t want = (total + kTrackThreads - 1) / kTrackThreads;
   if (want < (uint64_t)grid) grid = (int)want;
   const size_t threads = (size_t)grid * kTrackThreads;
   // workspace: the visit tables, the loopcheck tables (keys, then directions), the repacked samples

@@ -534,7 +534,7 @@ void bpx_track_options_default(bpx_track_options* opts);
  * and sample, and per particle in flight a visit table of 8 * 2^ceil(log2(2 * (nsteps + 2))) bytes
  * (twice that with matrix2), with loopcheck a coarse-cell table of 24 bytes per entry, and with avoid,
  * waypoints or distthresh lists of 4 * nsteps bytes (not where those options track particles twice: with
- * matrix2, or targets and distthresh); 1024 particles in flight per multiprocessor, or the call's own
+ * matrix2, with targets and distthresh, or where the tables leave room for few particles); 1024 particles in flight per multiprocessor, or the call's own
  * number if that is less, fewer if all this would pass 16 GB (5 GB on a B200 at nsteps 2000 without
  * options).
  */
