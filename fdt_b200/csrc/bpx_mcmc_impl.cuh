@@ -1022,12 +1022,16 @@ cudaError_t launch_mcmc_t(const McmcArgs& args, cudaStream_t s) {
     else if (!stretch && a.ndir >= 2 * NP * TPV)
       kern = mcmc_kernel<MODEL, K, RIC, TPV, MPL, false, 1>;
   }
-  const size_t smem = (size_t)(a.gradnonlin ? GPB : 1) * TPV * MPL * sizeof(float4) +
-                      (size_t)NP * kMcmcThreads * sizeof(float4) + (size_t)kMcmcThreads * sizeof(float2) +
-                      (size_t)(2 * NP + 1) * (K + 1) * kMcmcThreads * sizeof(float) + (size_t)GPB * NS * 8 +
-                      (size_t)GPB * kFsRows * K * sizeof(float);
+  const auto need = [](int tables) {
+    return (size_t)tables * TPV * MPL * sizeof(float4) + (size_t)NP * kMcmcThreads * sizeof(float4) +
+           (size_t)kMcmcThreads * sizeof(float2) + (size_t)(2 * NP + 1) * (K + 1) * kMcmcThreads * sizeof(float) +
+           (size_t)GPB * NS * 8 + (size_t)GPB * kFsRows * K * sizeof(float);
+  };
+  const size_t smem = need(a.gradnonlin ? GPB : 1);
   if (smem > 48 * 1024) {
-    cudaError_t ea = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the limit belongs to the process: set only ever to the larger need, so that no call lowers it for
+    // another one between its setting and its launch
+    cudaError_t ea = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need(GPB));
     if (ea != cudaSuccess) return ea;
   }
   int per_sm = 0;

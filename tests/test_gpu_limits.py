@@ -82,6 +82,31 @@ def test_fits_of_several_sizes_on_several_threads(torch):
             assert torch.equal(g.view(torch.int32), w.view(torch.int32))
 
 
+def test_chains_with_and_without_a_b_matrix_per_voxel_on_several_threads(torch):
+    """512 measurements of three fibres: 60 KB with one b-matrix for all voxels, 84 KB with one for each."""
+    from fdt_b200 import lib
+
+    L, ndir, n = lib.load(), 512, 3
+    y, bvecs, bvals = _voxels(ndir, n, 3)
+    d = lib.to_device(y)
+    tables = {0: (bvecs, bvals), 1: (np.tile(bvecs, (n, 1, 1)), np.tile(bvals, (n, 1)))}
+    calls, results, keep = [], [], []
+    for each in (0, 1, 0, 1):
+        o = Options.make(model=1, nfibres=3, gradnonlin=each, nburn=0, njumps=2, sampleevery=2)
+        bv, bl = (lib.to_device(a) for a in tables[each])
+        params, _, _ = lib.fit(o, d, bv, bl)
+        want = lib.mcmc(o, d, bv, bl, params)
+        got, vol = torch.zeros_like(want), lib.make_volume(d, bv, bl)
+        keep.append((o, bv, bl, params, vol))
+        results.append((got, want))
+        calls.append(lambda s, o=o, vol=vol, params=params, got=got: L.bpx_mcmc_dev(
+            C.byref(o), C.byref(vol), params.data_ptr(), None, got.data_ptr(), None, s))
+    torch.cuda.synchronize()
+    assert not _on_threads(torch, calls, 3000)
+    for got, want in results:
+        assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+
+
 def test_batch_of_several_sizes(torch):
     """The largest size is captured first, the smaller one after it."""
     from fdt_b200 import lib
