@@ -427,7 +427,7 @@ struct Stretch {
 
 bpx_status mcmc_run(const bpx_options* opts, const bpx_volume* vol, const float* params, const float* tau,
                     const float* props_in, float* props_out, int32_t freeze_props, float* records,
-                    uint32_t* status, void* stream, const Stretch* sp) {
+                    uint32_t* status, void* stream, const Stretch* sp, bool alone) {
   NvtxRange nvtx_range("bpx.mcmc");
   bpx_status st = check_opts(opts);
   if (st == BPX_OK) st = check_vol(vol, true);
@@ -472,6 +472,7 @@ bpx_status mcmc_run(const bpx_options* opts, const bpx_volume* vol, const float*
   a.props_out = props_out;
   if (freeze_props < 0 || freeze_props > 2) return fail(BPX_ERR_INVALID_ARG, "freeze_props must be 0, 1 or 2");
   a.freeze_props = freeze_props;
+  a.alone = alone;
   if (sp) {
     a.it_begin = sp->it_begin;
     a.it_end = sp->it_end;
@@ -485,6 +486,14 @@ bpx_status mcmc_run(const bpx_options* opts, const bpx_volume* vol, const float*
 }
 
 }  // namespace
+
+// The pipelines on the shared workspace run one after another (see Concurrency in bpx.h); those of a handle,
+// like the chains of direct calls and of batches, may run beside others.
+bpx_status api_pipeline_mcmc(const bpx_options* opts, const bpx_volume* vol, const float* params, const float* tau,
+                             const float* props_in, int32_t freeze_props, float* records, uint32_t* status, void* stream) {
+  return mcmc_run(opts, vol, params, tau, props_in, nullptr, freeze_props, records, status, stream, nullptr, !g_bound);
+}
+
 }  // namespace bpx
 
 extern "C" {
@@ -492,7 +501,7 @@ extern "C" {
 bpx_status bpx_mcmc_ex_dev(const bpx_options* opts, const bpx_volume* vol, const float* params, const float* tau,
                            const float* props_in, float* props_out, int32_t freeze_props, float* records,
                            uint32_t* status, void* stream) {
-  return mcmc_run(opts, vol, params, tau, props_in, props_out, freeze_props, records, status, stream, nullptr);
+  return mcmc_run(opts, vol, params, tau, props_in, props_out, freeze_props, records, status, stream, nullptr, false);
 }
 
 bpx_status bpx_mcmc_stretch_dev(const bpx_options* opts, const bpx_volume* vol, const float* params, const float* tau,
@@ -507,7 +516,7 @@ bpx_status bpx_mcmc_stretch_dev(const bpx_options* opts, const bpx_volume* vol, 
     return fail(BPX_ERR_INVALID_ARG, "need 0 <= it_begin < it_end <= nburn + njumps");
   if (it_begin > 0 && !state_in) return fail(BPX_ERR_INVALID_ARG, "a stretch that starts after iteration 0 needs state_in");
   Stretch sp{it_begin, it_end, state_in, state_out, acc_in, acc_out};
-  return mcmc_run(opts, vol, params, tau, props_in, props_out, freeze_props, records, status, stream, &sp);
+  return mcmc_run(opts, vol, params, tau, props_in, props_out, freeze_props, records, status, stream, &sp, false);
 }
 
 bpx_status bpx_mcmc_dev(const bpx_options* opts, const bpx_volume* vol, const float* params, const float* tau,
@@ -626,7 +635,7 @@ bpx_status bpx_xfibres_dev(const bpx_options* opts, const bpx_volume* vol, bpx_o
   }
   st = bpx_fit_dev(opts, vol, params, tau, status, stream);
   if (st != BPX_OK) return st;
-  st = bpx_mcmc_dev(opts, vol, params, tau, rec, status, stream);
+  st = api_pipeline_mcmc(opts, vol, params, tau, nullptr, 0, rec, status, stream);
   if (st != BPX_OK) return st;
   st = bpx_finish_dev(opts, vol->nvox, rec, out, stream);
   return st;

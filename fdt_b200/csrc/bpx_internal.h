@@ -62,6 +62,9 @@ bpx_status api_check_device();
 bpx_status api_check_opts(const bpx_options* o);
 bpx_status api_check_vol(const bpx_volume* v);
 bpx_status api_workspace(int slot, size_t bytes, void** out);
+// bpx_mcmc_ex_dev as a stage of a pipeline (no widths out)
+bpx_status api_pipeline_mcmc(const bpx_options* opts, const bpx_volume* vol, const float* params, const float* tau,
+                             const float* props_in, int32_t freeze_props, float* records, uint32_t* status, void* stream);
 // bpx_fit_dev with caller-provided stage scratch (nvox * kFitScratchBytes, 8-byte aligned)
 bpx_status fit_dev_scratch(const bpx_options* opts, const bpx_volume* vol, float* params, float* tau, uint32_t* status,
                            void* scratch, void* stream);
@@ -104,7 +107,8 @@ struct McmcArgs {
   const float* props_in;  // [6+3K][nvox] initial proposal widths, or NULL for initialise_props
   float* props_out;       // [6+3K][nvox] proposal widths after the last iteration, or NULL
   int freeze_props;       // 0: adapt (reference); 1: never adapt; 2: adapt during burn-in only
-  int spread;             // one voxel per warp whatever the layout (set by the launcher for small volumes)
+  int alone;              // the caller knows that no other chains run beside these (see launch_mcmc_t)
+  int spread;             // one voxel per warp whatever the layout (set by the launcher)
   const uint64_t* voxel_keys;  // [nvox] RNG voxel keys (packed batches), or NULL: voxel_offset + v
   // a stretch of the chain: iterations [it_begin, it_end) (it_end 0: to the end), started from
   // state_in [6+3K][nvox] (record rows) and acc_in [6+3K][nvox] when given; the state, acceptance

@@ -1006,10 +1006,17 @@ cudaError_t launch_mcmc_t(const McmcArgs& args, cudaStream_t s) {
   McmcArgs a = args;
   // A volume of no more voxels than the device has schedulers is bound by the latency of one warp's
   // chain, and the groups of a warp lengthen it by taking different branches (accept and restore, prior
-  // rejections): each warp then runs one voxel.  500 voxels, 64 measurements (8 lanes each): 12.6 ->
-  // 11.8 ms; with more voxels the warps share schedulers and it no longer pays (1000 voxels, 65
-  // measurements: 1.62 ms packed, 1.76 ms spread).
-  a.spread = TPV < 32 && a.nvox <= 4 * sm_count();
+  // rejections): each warp then runs one voxel, which its groups repeat.
+  //   chains of 500 voxels, 2250 iterations   packed   spread ms
+  //   33 measurements, model 1, 2 fibres       13.45    12.62      (4 lanes a voxel)
+  //   64                                       12.58    11.75      (8)
+  //   129                                      12.65    12.17      (16)
+  //   129, model 2, 3 fibres, Rician           29.9     26.2
+  // More voxels would share schedulers, and so do chains that run beside these, whose warps then number
+  // two to eight times as many: 2, 4 and 8 streams of the 64-measurement chains take 12.6, 12.6, 14.4 ms
+  // packed and 13.5, 18.2, 32.3 ms spread, a batch of nine buckets of 590 voxels 109 and 238 ms.  So
+  // chains are spread only where the caller knows that they are alone.
+  a.spread = a.alone && TPV < 32 && a.nvox <= 4 * sm_count();
   const bool stretch = a.it_begin != 0 || a.it_end != 0 || a.state_in || a.state_out || a.acc_in || a.acc_out;
   constexpr int NS = 6 + 3 * K, GPB = kMcmcThreads / TPV;
   constexpr int NP = MPL / 2;

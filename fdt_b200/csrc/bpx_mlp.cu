@@ -751,8 +751,7 @@ bpx_status bpx_xfibres_learned_dev(const bpx_options* opts, const bpx_volume* vo
   if (st == BPX_OK) st = bpx_mlp_forward_dev(vol->ndir, mlp_params, vol->nvox, x, netout, stream);
   if (st == BPX_OK) st = bpx_mlp_decode_dev(opts, vol->nvox, netout, s0hat, params, tau, props, status, stream);
   if (st == BPX_OK)
-    st = bpx_mcmc_ex_dev(opts, vol, params, opts->rician ? tau : nullptr, props, nullptr, freeze_props, rec, status,
-                         stream);
+    st = api_pipeline_mcmc(opts, vol, params, opts->rician ? tau : nullptr, props, freeze_props, rec, status, stream);
   if (st == BPX_OK) st = bpx_finish_dev(opts, vol->nvox, rec, out, stream);
   return st;
 }
