@@ -37,6 +37,7 @@
 
 #include "bpx_gemm.h"
 #include "bpx_internal.h"
+#include "bpx_ring.h"
 
 namespace bpx {
 namespace gemm {
@@ -208,53 +209,47 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_kernel(const __grid_constant
   if (threadIdx.x == 0) {
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)g.a_mn << 15) | ((uint32_t)g.b_mn << 16) |
                            ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
-    auto load = [&](int kc, int s) {
-      const uint32_t sa = smem_u32(base + s * stage_bytes), sb = sa + a_bytes;
-      const uint32_t bar = smem_u32(&sm->full[s]);
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" : : "r"(bar), "r"(stage_bytes) : "memory");
-      if (g.a_mn)
-        for (int j = 0; j < kTileM / kSpan; ++j)
-          tma_load_2d(sa + j * kSpan * kChunkK * 2, &map_a, m0 + j * kSpan, kc * kChunkK, bar);
-      else
-        tma_load_2d(sa, &map_a, kc * kChunkK, m0, bar);
-      if (g.b_mn)
-        for (uint32_t j = 0; j * kSpan * kChunkK * 2 < b_bytes; ++j)
-          tma_load_2d(sb + j * kSpan * kChunkK * 2, &map_b, n0 + j * kSpan, kc * kChunkK, bar);
-      else
-        tma_load_2d(sb, &map_b, kc * kChunkK, n0, bar);
-    };
-    bool ok = true;
-    for (int i = 0; i < stages && kc0 + i < kc1; ++i) load(kc0 + i, i);
-    int s = 0;
-    uint32_t ph = 0;
-    for (int kc = kc0; kc < kc1; ++kc) {
-      if (!mbar_wait(smem_u32(&sm->full[s]), ph)) {
-        ok = false;
-        break;
+    struct Ops {
+      const GemmArgs& g;
+      const CUtensorMap &map_a, &map_b;
+      Smem* sm;
+      uint32_t base, a_bytes, b_bytes, tmem, idesc;
+      int m0, n0, kc0;
+      __device__ __forceinline__ uint32_t place(int s) const { return base + (uint32_t)s * (a_bytes + b_bytes); }
+      __device__ __forceinline__ void copy(int c, int s) const {
+        const uint32_t sa = place(s), sb = sa + a_bytes;
+        const uint32_t bar = smem_u32(&sm->full[s]);
+        const int k = (kc0 + c) * kChunkK;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" : : "r"(bar), "r"(a_bytes + b_bytes) : "memory");
+        if (g.a_mn)
+          for (int j = 0; j < kTileM / kSpan; ++j) tma_load_2d(sa + j * kSpan * kChunkK * 2, &map_a, m0 + j * kSpan, k, bar);
+        else
+          tma_load_2d(sa, &map_a, k, m0, bar);
+        if (g.b_mn)
+          for (uint32_t j = 0; j * kSpan * kChunkK * 2 < b_bytes; ++j)
+            tma_load_2d(sb + j * kSpan * kChunkK * 2, &map_b, n0 + j * kSpan, k, bar);
+        else
+          tma_load_2d(sb, &map_b, k, n0, bar);
       }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t sa = smem_u32(base + s * stage_bytes), sb = sa + a_bytes;
+      __device__ __forceinline__ bool wait_full(int s, uint32_t ph) const { return mbar_wait(smem_u32(&sm->full[s]), ph); }
+      __device__ __forceinline__ bool wait_empty(int s, uint32_t ph) const { return mbar_wait(smem_u32(&sm->empty[s]), ph); }
+      __device__ __forceinline__ void drain(int s, uint32_t ph) const { mbar_wait(smem_u32(&sm->full[s]), ph); }
+      __device__ __forceinline__ void multiply(int c, int s) const {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t sa = place(s), sb = sa + a_bytes;
 #pragma unroll
-      for (int ks = 0; ks < kChunkK / 16; ++ks) {
-        const uint64_t da = g.a_mn ? smem_desc(sa + ks * 2048, kSpan * kChunkK * 2, 1024) : smem_desc(sa + ks * 32, 0, 1024);
-        const uint64_t db = g.b_mn ? smem_desc(sb + ks * 2048, kSpan * kChunkK * 2, 1024) : smem_desc(sb + ks * 32, 0, 1024);
-        mma_bf16(tmem, da, db, idesc, (kc != kc0) || ks != 0);
-      }
-      mma_commit(smem_u32(&sm->empty[s]));
-      if (kc + stages < kc1) {
-        if (!mbar_wait(smem_u32(&sm->empty[s]), ph)) {
-          ok = false;
-          break;
+        for (int ks = 0; ks < kChunkK / 16; ++ks) {
+          const uint64_t da = g.a_mn ? smem_desc(sa + ks * 2048, kSpan * kChunkK * 2, 1024) : smem_desc(sa + ks * 32, 0, 1024);
+          const uint64_t db = g.b_mn ? smem_desc(sb + ks * 2048, kSpan * kChunkK * 2, 1024) : smem_desc(sb + ks * 32, 0, 1024);
+          mma_bf16(tmem, da, db, idesc, c != 0 || ks != 0);
         }
-        load(kc + stages, s);
+        mma_commit(smem_u32(&sm->empty[s]));
       }
-      if (++s == stages) {
-        s = 0;
-        ph ^= 1;
-      }
-    }
-    if (!ok && g.error) atomicExch(g.error, 1);
-    mma_commit(smem_u32(&sm->done));  // arrives once every MMA issued above has completed
+      // arrives once every MMA issued has completed
+      __device__ __forceinline__ void finish() const { mma_commit(smem_u32(&sm->done)); }
+    };
+    const Ops ops{g, map_a, map_b, sm, smem_u32(base), a_bytes, b_bytes, tmem, idesc, m0, n0, kc0};
+    if (!ring_contract(ops, kc1 - kc0, stages) && g.error) atomicExch(g.error, 1);
   }
   __syncwarp();
   const bool done = mbar_wait(smem_u32(&sm->done), 0);
@@ -467,50 +462,34 @@ __device__ __forceinline__ bool chain_wait(ChainBars* sm, const uint64_t* bar, u
   return true;
 }
 
-// Pieces come in order of use: layer, chunk of K, half of the columns (the last layer, of kChainOut
-// columns, has one).  Piece p takes ring slot p % kRing.  One thread copies, another multiplies: a single
-// one, which also divided for slots and rounds, took 1300 cycles a piece, 3000 beside busy epilogue
-// warps, and was the kernel's bound (205 us for the 65536 rows).
-__device__ __forceinline__ int chain_chunks(int layer, int nk0) { return layer == 0 ? nk0 : kActSpans; }
-__device__ __forceinline__ int chain_halves(int layer) { return layer == kChainLayers - 1 ? 1 : kChainWidth / kPieceN; }
+// One thread copies the pieces, another multiplies: a single one, which also divided for slots and rounds,
+// took 1300 cycles a piece, 3000 beside busy epilogue warps, and was the kernel's bound (205 us for the
+// 65536 rows).  The last layer's pieces have kChainOut columns.
+using ChainRing = RingChain<kChainLayers, kActSpans, kRing, kChainWidth / kPieceN>;
 
-__device__ __forceinline__ bool chain_copy(const Chain& c, ChainBars* sm, uint32_t act, uint32_t ring, int m0, int nk0,
-                                           int* copied) {
-  int p = 0, slot = 0;
-  uint32_t ph = 1;  // of the slot's previous piece; the first round finds its slots empty
-  for (int layer = 0; layer < kChainLayers; ++layer) {
-    const int halves = chain_halves(layer), nk = chain_chunks(layer, nk0);
-    const uint32_t w_bytes = halves == 1 ? kChainOut * kChunkK * 2 : kSpanBytes;
-    for (int kc = 0; kc < nk; ++kc)
-      for (int half = 0; half < halves; ++half) {
-        *copied = p;
-        if (p >= kRing && !chain_wait(sm, &sm->empty[slot], ph)) return false;
-        const bool with_x = layer == 0 && half == 0;
-        if (with_x && kc >= kActSpans) {  // the chunk that was in this span
-          const int q = p - 2 * kActSpans + 1;
-          if (!chain_wait(sm, &sm->empty[q % kRing], (q / kRing) & 1)) return false;
-        }
-        const uint32_t bar = smem_u32(&sm->full[slot]), bytes = w_bytes + (with_x ? kSpanBytes : 0);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" : : "r"(bar), "r"(bytes) : "memory");
-        if (with_x) tma_load_2d(act + (kc % kActSpans) * kSpanBytes, &c.x, kc * kChunkK, m0, bar);
-        tma_load_2d(ring + slot * kSpanBytes, &c.w[layer], kc * kChunkK, half * kPieceN, bar);
-        ++p;
-        if (++slot == kRing) {
-          slot = 0;
-          ph ^= 1;
-        }
-      }
+struct ChainCopy {
+  const Chain& c;
+  ChainBars* sm;
+  uint32_t act, ring;
+  int m0;
+  __device__ __forceinline__ bool wait_empty(int slot, uint32_t ph) const { return chain_wait(sm, &sm->empty[slot], ph); }
+  __device__ __forceinline__ void drain(int slot, uint32_t ph) const { mbar_wait(smem_u32(&sm->full[slot]), ph); }
+  __device__ __forceinline__ void copy(int layer, int kc, int half, int slot) const {
+    const bool with_x = layer == 0 && half == 0;
+    const uint32_t w_bytes = ChainRing::halves(layer) == 1 ? kChainOut * kChunkK * 2 : kSpanBytes;
+    const uint32_t bar = smem_u32(&sm->full[slot]), bytes = w_bytes + (with_x ? kSpanBytes : 0);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" : : "r"(bar), "r"(bytes) : "memory");
+    if (with_x) tma_load_2d(act + (kc % kActSpans) * kSpanBytes, &c.x, kc * kChunkK, m0, bar);
+    tma_load_2d(ring + slot * kSpanBytes, &c.w[layer], kc * kChunkK, half * kPieceN, bar);
   }
-  *copied = p;
-  return true;
-}
+};
 
 __device__ __forceinline__ bool chain_multiply(ChainBars* sm, uint32_t act, uint32_t ring, uint32_t tmem, int nk0) {
   int slot = 0;
   uint32_t ph = 0;
   const uint64_t act_desc = smem_desc(act, 0, 1024), ring_desc = smem_desc(ring, 0, 1024);
   for (int layer = 0; layer < kChainLayers; ++layer) {
-    const int halves = chain_halves(layer), nk = chain_chunks(layer, nk0), n = halves == 1 ? kChainOut : kPieceN;
+    const int halves = ChainRing::halves(layer), nk = ChainRing::chunks(layer, nk0), n = halves == 1 ? kChainOut : kPieceN;
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
     const uint32_t sums = tmem + (layer & 1) * kChainWidth;
     for (int kc = 0; kc < nk; ++kc) {
@@ -572,16 +551,14 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_kernel(const __grid_co
 
   const int nk0 = (c.nin + kChunkK - 1) / kChunkK;
   if (warp == kEpiWarps) {
-    int copied = 0;
-    if (lane == 0 && !chain_copy(c, sm, smem_u32(act), smem_u32(ring), m0, nk0, &copied)) {
-      // the copies in flight end before the shared memory goes
-      for (int p = copied > kRing ? copied - kRing : 0; p < copied; ++p)
-        mbar_wait(smem_u32(&sm->full[p % kRing]), (p / kRing) & 1);
+    if (lane == 0) {
+      const ChainCopy ops{c, sm, smem_u32(act), smem_u32(ring), m0};
+      ChainRing::copy(ops, nk0);
     }
     __syncwarp();
   } else if (warp == kEpiWarps + 1) {
     if (lane == 0 && !chain_multiply(sm, smem_u32(act), smem_u32(ring), tmem, nk0)) {
-      mma_commit(smem_u32(&sm->drained));  // and so do the products
+      mma_commit(smem_u32(&sm->drained));  // the products in flight end before the shared memory goes
       mbar_wait(smem_u32(&sm->drained), 0);
     }
     __syncwarp();
