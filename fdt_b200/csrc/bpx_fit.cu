@@ -1159,8 +1159,8 @@ __device__ void stage_finish(const FitArgs& a, int v, int lane, double*) {
 // The warps of a resident grid take voxels from the launch's counter (queue, zero before it) as they
 // finish, so a voxel whose fit runs 200 iterations holds up one warp and a volume of any size spreads
 // over every SM.  (With 32 consecutive voxels shared out inside each block, a volume of a few
-// thousand voxels left SMs idle or doubly loaded: 8192 / 12800 whole-brain voxels took 206 / 245 ms,
-// with the launch-wide counter 133 / 187 ms.)
+// thousand voxels left SMs idle or doubly loaded: 8192 / 12800 / 32768 whole-brain voxels took 207 / 236 /
+// 507 ms, with the launch-wide counter 131 / 170 / 419 ms.)
 template <typename Stage>
 __device__ __forceinline__ void run_stage(const FitArgs& a, unsigned int* queue, Stage stage) {
   __shared__ double stage_buf[kFitThreads / 32][kStageDoubles];

@@ -9,7 +9,10 @@
 //     formed once per distinct b-value and trial (BTable), one lane each, not once per measurement;
 //   * sines, cosines and arctangents of the parameters are formed one per lane, not all in every lane;
 //   * parameters live one per lane and the point's constants in shared memory, which leaves registers
-//     for kFitStartMinBlocks blocks per SM.
+//     for kFitStartMinBlocks blocks per SM.  Shared memory, K values per measurement and warp, leaves room
+//     for them up to 333 measurements of three fibres, for four blocks up to 454 and for three at 512, where
+//     the register form had four; model 1 fits of 4000 voxels of 512 measurements take 22.8 ms all the same
+//     (55.0 in the register form with a counter per block), of 288 measurements 11.9 (36.2).
 // Every value is formed by the operations, in the order, of the register form (bpx_fit.cu), and the fits
 // are equal bit for bit.  The first fit of 12800 whole-brain voxels took 32.4 ms in the register form.
 // PVM_multi keeps that form: with two and three fibres its normal equations are so ill-conditioned that

@@ -19,7 +19,7 @@
 // an mbarrier ring of two to four stages; eight warps then read the accumulator (tcgen05.ld: warp w
 // the 32 TMEM lanes w%4, every second block of 32 columns) and run the epilogue.  Every mbarrier
 // wait is bounded (about a second), after which the kernel records an error code, waits (bounded) for
-// its own MMAs and releases its tensor memory.
+// its own copies and MMAs and releases its tensor memory (bpx_ring.h).
 //
 // The network's contractions are 2 to 5 chunks deep, so most of a CTA's time is its epilogue (256 erff per
 // row of a 256-wide tile): bound by FP32 issue and by the loads that precede it, not by the tensor pipe.  Hence eight

@@ -586,10 +586,12 @@ bpx_status bpx_mlp_train_step_dev(int32_t ndir, const float* params, float* grad
   const size_t B = (size_t)batch;
   const size_t b_w = a256(G.nw * 2), b_a = a256(B * kWidth * 2), b_z = a256(B * kWidth * 4);
   const size_t b_out = a256(B * kOut * 4), b_dz5 = a256(B * kOut * 2);
-  // the weight gradients' outputs are a few tiles each with the whole batch to contract: 32-column
-  // tiles of all layers in one launch, each contraction in two parts, give every SM a CTA at 4096
-  // rows.  (Eight parts are no faster end to end and move the sums, whose
-  // accumulation the tensor core rounds, nearer to 1e-5 from the undivided ones.)
+  // the weight gradients' outputs are a few tiles each with the whole batch to contract: 128 x 32 tiles of
+  // all layers in one launch, each contraction in two parts, are 2 x 74 CTAs for 288 inputs, one for each of
+  // 148 SMs, and 120 to 176 for 33 to 512.  Both numbers are constants: tiles come no narrower, and the
+  // parts set the order of the sums, which is to depend on the batch alone.  (Eight parts are no faster end
+  // to end and move the sums, whose accumulation the tensor core rounds, nearer to 1e-5 from the undivided
+  // ones.)
   const int chunks = (batch + 63) / 64;
   const int splits = chunks >= 16 ? 2 : 1;
   const size_t b_part = a256(G.nw * splits * 4);
